@@ -9,7 +9,6 @@
 #include <functional>
 #include <map>
 #include <mutex>
-#include <queue>
 #include <type_traits>
 #include <string>
 #include <vector>
@@ -144,7 +143,6 @@ struct amdk_ctx {
   };
   std::map<std::array<int, 4>, SegGraph> graphs;
   bool use_graphs = true;
-  bool tune = true;  // measure launch shapes at first use (AMDK_NO_TUNE=1: model only)
   bool overlap = true;  // C0-only work on the side stream (AMDK_NO_OVERLAP=1: one stream)
   // integer-slice tensor-core GEMMs of the mixed path (<= 128 bands;
   // AMDK_NO_SLICE=1: DGEMM/DTRMM as the FP64 path)
@@ -178,22 +176,14 @@ struct amdk_ctx {
   double pred_coef[MAX_PRED] = {2.0, -1.0};       // weights of C0(t), C0(t-dt), ...
   bool pred_user = false;                         // coefficients given by the caller
   int *h_info = nullptr;    // pinned: Cholesky status
-  int pencil_groups = 1;  // upper bound on the density pair groups
-  int ct_vpsi = 0, ct_dens = 0;  // column tiles of the pencil kernels (current precision)
-  int ns_dens = 1;               // register slots of the density kernel's sums (tiles x task rounds)
-  int nsd_p[2] = {1, 1};
   bool pv_p[2] = {false, false}, pd_p[2] = {false, false};  // per pair precision: FP64, mixed
-  int ctv_p[2] = {0, 0}, ctd_p[2] = {0, 0};
-  int pn1 = 0, pn2 = 0;          // two-level split n = pn1 * pn2
   int nsm = 148;
   // one resident wave of the streaming reductions (blocks per SM x SMs)
   int red_ekin = RED_BLOCKS, red_gmax = RED_BLOCKS;
-  std::map<int, int> pencil_grp_cache;
-  int vpsi_tuned[2] = {0, 0};  // batch size the V(r)psi column tile was measured for, per precision
   PencilGeom pg{};
-  int *d_rpos = nullptr, *d_gmapt = nullptr, *d_zinv = nullptr, *d_postp = nullptr, *d_postm = nullptr;
+  int *d_cols = nullptr, *d_gmapt = nullptr, *d_postp = nullptr, *d_postm = nullptr;
   double *d_rhopart = nullptr;
-  void *d_vt = nullptr;
+  void *d_vt = nullptr, *d_pscr = nullptr;  // permuted V; shares of rays between column groups (VpsiShape::GA > 1)
   // live per-kernel timing (CUDA events on the context stream)
   long nlaunch = 0;  // kernels of this library launched on the context stream
   bool prof = false;
@@ -432,80 +422,40 @@ static int grid_to_rays(amdk_ctx *c, int T, const double2 *cgrid, const double *
 }
 
 // ------------------------------------------------------------------ pencil path
-// shared memory of a pencil block: slab plane, column tile of ct columns,
-// the twiddle tables (2n, from a 16-byte boundary) and the packed slab-plane
-// table (16 bytes for each of at most 16 j2)
-template <typename C> static size_t pencil_smem(int n, int nz, int ct) {
-  return (((size_t)(nz + ct) * (n + 1) * sizeof(C) + 15) & ~(size_t)15) + 2 * (size_t)n * sizeof(C) + 16 * 16;
-}
-// widest column tile with the block within `budget` bytes (0: none fits)
-template <typename C> static int pencil_tile(int n, int nz, size_t extra, size_t budget) {
-  const size_t base = pencil_smem<C>(n, nz, 0) + extra;
-  if (base >= budget) return 0;
-  const int widest = (int)std::min<size_t>(n, (budget - base) / ((n + 1) * sizeof(C)));
-  if (widest <= 0) return 0;
-  const int tiles = (n + widest - 1) / widest;  // equal tiles
-  return (n + tiles - 1) / tiles;
-}
-// Column tiles of the density pencil kernel: the fewest equal tiles (1, 2 or
-// 4) whose block fits the shared memory of two blocks per SM (else of one),
-// whose group sums fit 1, 2 or 4 register slots (tiles x rounds of PNT
-// tasks) and whose final staging of the sums (n x (n+1) reals) fits over the
-// plane and the tile.  ct = 0 when none does.
-static void density_tiles(int n, int nz, size_t csize, size_t lim, int *ct, int *ns) {
-  *ct = 0;
-  *ns = 1;
-  const int n1f = fft_n1(n);
-  for (size_t budget : {lim / 2, lim})
-    for (int tiles : {1, 2, 4}) {
-      const int w = (n + tiles - 1) / tiles;
-      const size_t smem = (((size_t)(nz + w) * (n + 1) * csize + 15) & ~(size_t)15) + 2 * (size_t)n * csize + 16 * 16;
-      const int reps = (w * n1f + PNT - 1) / PNT;
-      const int slots = tiles * reps;
-      const bool stage_ok = (size_t)n * (n + 1) * (csize / 2) <= (size_t)(nz + w) * (n + 1) * csize;
-      if (smem <= budget && stage_ok && (slots == 1 || slots == 2 || slots == 4) && (n + w - 1) / w == tiles) {
-        *ct = w;
-        *ns = slots;
-        return;
+// elements of the ray buffer per pair on the pencil path
+static long pencil_stride(const amdk_ctx *c) { return (long)c->pg.nray * c->geom.n1; }
+// the twiddle tables of a length, a kernel parameter
+template <typename C, int N> static const PencilTw<C, N> &pencil_tw() {
+  static const PencilTw<C, N> t = []() {
+    PencilTw<C, N> x;
+    constexpr int N1 = fft_n1(N), N2 = N / N1;
+    const double tp = 8.0 * std::atan(1.0);
+    for (int i = 0; i < N; ++i)
+      for (int h = 0; h < 2; ++h) {
+        const int d = h ? N2 : N1, e = (i / d) * (i % d) % N;
+        const double a = -tp * (double)e / (double)N;
+        x.t[h * N + i].x = (decltype(x.t[0].x))std::cos(a);
+        x.t[h * N + i].y = (decltype(x.t[0].x))std::sin(a);
       }
-    }
+    return x;
+  }();
+  return t;
+}
+// resident blocks per SM of a pencil kernel
+template <auto K> static int pencil_resident(int nt, size_t smem) {
+  static const int nb = [&]() {
+    smem_opt_in<K>();
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, K, nt, smem) != cudaSuccess) n = 0;
+    cudaGetLastError();
+    return std::max(n, 1);
+  }();
+  return nb;
 }
 template <typename C> static size_t xt_smem(int n1) { return ((size_t)XL * (n1 + 1) + 2 * n1) * sizeof(C); }
-// Pair groups of the density pencil kernel: each (x-plane, group) block sums
-// its group's pairs into its own partial grid.  Pick the group count whose
-// block list, scheduled greedily on the SMs, ends first; each group also
-// costs one partial grid written and read back.
-static int pencil_density_groups(int n1, int T, int nsm, int bps, int maxg) {
-  int best = 1;
-  double best_cost = 1e300;
-  for (int grp = 1; grp <= std::min(maxg, T); ++grp) {
-    const int per = (T + grp - 1) / grp;
-    if ((grp - 1) * per >= T) continue;  // an empty group
-    std::priority_queue<double, std::vector<double>, std::greater<double>> slots;
-    for (int i = 0; i < nsm * bps; ++i) slots.push(0.0);
-    double end = 0.0;
-    for (int gi = 0; gi < grp; ++gi) {
-      const int np = std::min(T, (gi + 1) * per) - gi * per;
-      for (int kx = 0; kx < n1; ++kx) {
-        double t0 = slots.top();
-        slots.pop();
-        double t1 = t0 + (np + 0.5) / bps;
-        end = std::max(end, t1);
-        slots.push(t1);
-      }
-    }
-    const double cost = end + 0.3 * grp;
-    if (cost < best_cost) {
-      best_cost = cost;
-      best = grp;
-    }
-  }
-  return best;
-}
-
 template <typename C> static void xt_bwd_pair(amdk_ctx *c, int p0, int T) {
   const Geom &g = c->geom;
-  long lines = (long)T * g.nray[0];
+  long lines = (long)T * c->pg.nray;
   with_n(g.n1, [&](auto NC) {
     constexpr int N = decltype(NC)::value;
     if constexpr (N > 0) {
@@ -519,7 +469,7 @@ template <typename C> static void xt_bwd_pair(amdk_ctx *c, int p0, int T) {
 }
 template <typename C> static void xt_fwd(amdk_ctx *c, int T) {
   const Geom &g = c->geom;
-  long lines = (long)T * g.nray[0];
+  long lines = (long)T * c->pg.nray;
   prof_begin(c, KT_X, 2.0 * lines * g.n1 * sizeof(C));
   with_n(g.n1, [&](auto NC) {
     constexpr int N = decltype(NC)::value;
@@ -532,147 +482,32 @@ template <typename C> static void xt_fwd(amdk_ctx *c, int T) {
   });
   prof_end(c);
 }
-// ------------------------------------------------------------------ tuning
-// Launch shapes measured at first use (AMDK_NO_TUNE=1: the model's choice
-// instead) are kept per context and, when AMDK_TUNE_CACHE names a file, in
-// that JSON object of "key": value pairs (keys name the kernel, precision,
-// grid, slab planes and batch), so that later contexts and processes reuse
-// them without measuring.
-static std::mutex g_tune_mu;
-static std::map<std::string, int> g_tune;
-static bool g_tune_loaded = false;
-static const char *tune_path() {
-  const char *p = getenv("AMDK_TUNE_CACHE");
-  return (p && *p) ? p : nullptr;
-}
-static void tune_load_locked() {
-  if (g_tune_loaded) return;
-  g_tune_loaded = true;
-  const char *path = tune_path();
-  if (!path) return;
-  FILE *f = std::fopen(path, "r");
-  if (!f) return;
-  std::string txt;
-  char buf[4096];
-  size_t nr;
-  while ((nr = std::fread(buf, 1, sizeof(buf), f)) > 0) txt.append(buf, nr);
-  std::fclose(f);
-  size_t i = 0;
-  while ((i = txt.find('"', i)) != std::string::npos) {
-    const size_t j = txt.find('"', i + 1);
-    if (j == std::string::npos) break;
-    const size_t k = txt.find(':', j);
-    if (k == std::string::npos) break;
-    g_tune[txt.substr(i + 1, j - i - 1)] = (int)std::strtol(txt.c_str() + k + 1, nullptr, 10);
-    i = txt.find_first_of(",}", k);
-    if (i == std::string::npos) break;
-  }
-}
-static bool tune_get(const std::string &key, int *v) {
-  std::lock_guard<std::mutex> lock(g_tune_mu);
-  tune_load_locked();
-  auto it = g_tune.find(key);
-  if (it == g_tune.end()) return false;
-  *v = it->second;
-  return true;
-}
-static void tune_put(const std::string &key, int v) {
-  std::lock_guard<std::mutex> lock(g_tune_mu);
-  tune_load_locked();
-  g_tune[key] = v;
-  const char *path = tune_path();
-  if (!path) return;
-  const std::string tmp = std::string(path) + ".tmp";
-  FILE *f = std::fopen(tmp.c_str(), "w");
-  if (!f) return;
-  std::fprintf(f, "{\n");
-  size_t n = 0;
-  for (auto &kv : g_tune) std::fprintf(f, "  \"%s\": %d%s\n", kv.first.c_str(), kv.second, ++n < g_tune.size() ? "," : "");
-  std::fprintf(f, "}\n");
-  std::fclose(f);
-  std::rename(tmp.c_str(), path);
-}
-// key of a tuned pencil launch shape
-static std::string pencil_key(const amdk_ctx *c, const char *what, int T) {
-  const Geom &g = c->geom;
-  return std::string(what) + "/" + (c->precision == AMDK_MIXED ? "mixed" : "fp64") + "/" + std::to_string(g.n1) + "x" +
-         std::to_string(g.n2) + "x" + std::to_string(g.n3) + "/nz" + std::to_string(c->pg.nz) + "/T" + std::to_string(T);
-}
-
-// pairs [p0, p0 + T) of the ray buffer rb; open shell: each pair with its
-// spin's potential (the pair straddling the spins with both)
-template <typename C, int N> static void launch_pencil_vpsi(amdk_ctx *c, int T, int ct, C *rb, int p0 = 0) {
+// V(r)psi on T pairs of nplane x planes (pg's buffer rb), one wave of
+// persistent blocks
+template <typename C, int N, bool SEG, bool LSD>
+static void launch_pencil_vpsi(int nsm, const PencilGeom &pg, C *rb, const void *vt, int T, void *scratch,
+                               const void *vt2, int gp0, int psplit, int pstraddle, cudaStream_t st) {
   typedef decltype(C().x) Rl;
-  const size_t sm = pencil_smem<C>(N, c->pg.nz, ct);
-  ++c->nlaunch;
-  if (c->hs.lsd) {
-    const int nu = c->hs.nel_up, psplit = (nu + 1) / 2, pstr = (nu & 1) ? nu / 2 : -1;
-    smem_opt_in<k_pencil_vpsi<C, N, true>>();
-    k_pencil_vpsi<C, N, true><<<dim3(c->geom.n1, T), PNT, sm, c->st>>>(
-        c->pg, plan<C>(c, 1), rb, (const Rl *)c->d_vt, ct, (const Rl *)c->d_vt2, p0, psplit, pstr);
-  } else {
-    smem_opt_in<k_pencil_vpsi<C, N>>();
-    k_pencil_vpsi<C, N><<<dim3(c->geom.n1, T), PNT, sm, c->st>>>(c->pg, plan<C>(c, 1), rb, (const Rl *)c->d_vt, ct,
-                                                                nullptr, 0, 0, -1);
-  }
+  typedef VpsiShape<C, N> Sh;
+  constexpr auto K = k_pencil_vpsi<C, N, SEG, LSD>;
+  const int units = pg.n1 * T, grid = std::min(units, nsm * pencil_resident<K>(Sh::NT, Sh::smem));
+  K<<<grid, Sh::NT, Sh::smem, st>>>(pg, pencil_tw<C, N>(), rb, (const Rl *)vt, units, (C *)scratch, (const Rl *)vt2, gp0,
+                                    psplit, pstraddle);
 }
-// Column-tile width of the V(r)psi pencil kernel for T pairs: measured once
-// per shape (every width ceil(N/t), t = 1..6, whose block fits, launched on a
-// scratch copy of the ray buffer, which the kernel transforms in place),
-// from the tuning cache, or the model's choice (capture, AMDK_NO_TUNE=1).
-template <typename C, int N> static int vpsi_tile(amdk_ctx *c, int T) {
-  const std::string key = pencil_key(c, "pencil_vpsi_tile", T);
-  const int q = (c->precision == AMDK_MIXED) ? 1 : 0;
-  int best = c->ctv_p[q];
-  if (c->vpsi_tuned[q] == T) return best;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  cudaStreamIsCapturing(c->st, &cap);
-  if (cap != cudaStreamCaptureStatusNone || !c->tune) return best;
-  int cached = 0;
-  if (tune_get(key, &cached) && cached >= 8 && pencil_smem<C>(N, c->pg.nz, cached) <= 227 * 1024) {
-    best = cached;
-  } else {
-    const size_t bytes = (size_t)T * rstride(c, 0) * sizeof(C);
-    C *scratch = nullptr;
-    if (cudaMalloc(&scratch, bytes) == cudaSuccess) {
-      cudaMemcpyAsync(scratch, c->d_rb, bytes, cudaMemcpyDeviceToDevice, c->st);
-      cudaEvent_t e0, e1;
-      cudaEventCreate(&e0);
-      cudaEventCreate(&e1);
-      const long nl = c->nlaunch;
-      float best_ms = 1e30f;
-      int prev = 0;
-      for (int t = 1; t <= 6; ++t) {
-        const int w = (N + t - 1) / t;
-        if (w == prev || w < 8 || pencil_smem<C>(N, c->pg.nz, w) > 227 * 1024) continue;
-        prev = w;
-        launch_pencil_vpsi<C, N>(c, T, w, scratch);  // warm
-        cudaEventRecord(e0, c->st);
-        launch_pencil_vpsi<C, N>(c, T, w, scratch);
-        launch_pencil_vpsi<C, N>(c, T, w, scratch);
-        cudaEventRecord(e1, c->st);
-        cudaEventSynchronize(e1);
-        float ms = 0;
-        cudaEventElapsedTime(&ms, e0, e1);
-        if (ms < best_ms) {
-          best_ms = ms;
-          best = w;
-        }
-      }
-      cudaEventDestroy(e0);
-      cudaEventDestroy(e1);
-      cudaStreamSynchronize(c->st);
-      cudaFree(scratch);
-      c->nlaunch = nl;  // tuning launches are not part of the work
-      tune_put(key, best);
+// bytes of the ray shares between column groups of launch_pencil_vpsi (0: not used)
+template <typename C> static size_t vpsi_scratch_bytes(int n, int nsm) {
+  size_t b = 0;
+  with_n(n, [&](auto NC) {
+    constexpr int N = decltype(NC)::value;
+    if constexpr (N > 0) {
+      constexpr size_t nz = Sphere<N>::NZ;
+      if (VpsiShape<C, N>::GA > 1) b = (size_t)nsm * VpsiShape<C, N>::MINB * nz * nz * sizeof(C);
     }
-    cudaGetLastError();
-  }
-  c->ctv_p[q] = best;
-  c->ct_vpsi = best;
-  c->vpsi_tuned[q] = T;
-  return best;
+  });
+  return b;
 }
+// pairs [p0, p0 + T) of the context's ray buffer; open shell: each pair with
+// its spin's potential (the pair straddling the spins with both)
 template <typename C> static void pencil_vpsi(amdk_ctx *c, int T, int p0 = 0) {
   const Geom &g = c->geom;
   typedef decltype(C().x) Rl;
@@ -680,135 +515,59 @@ template <typename C> static void pencil_vpsi(amdk_ctx *c, int T, int p0 = 0) {
   with_n(g.n2, [&](auto NC) {
     constexpr int N = decltype(NC)::value;
     if constexpr (N > 0) {
-      const int ct = vpsi_tile<C, N>(c, T);
-      prof_begin(c, KT_ZVPSI, 2.0 * T * rstride(c, 0) * sizeof(C) + npt * sizeof(Rl));
-      launch_pencil_vpsi<C, N>(c, T, ct, (C *)c->d_rb, p0);
+      prof_begin(c, KT_ZVPSI, 2.0 * T * pencil_stride(c) * sizeof(C) + npt * sizeof(Rl));
+      ++c->nlaunch;
+      if (c->hs.lsd) {
+        const int nu = c->hs.nel_up, psplit = (nu + 1) / 2, pstr = (nu & 1) ? nu / 2 : -1;
+        launch_pencil_vpsi<C, N, false, true>(c->nsm, c->pg, (C *)c->d_rb, c->d_vt, T, c->d_pscr, c->d_vt2, p0, psplit,
+                                              pstr, c->st);
+      } else {
+        launch_pencil_vpsi<C, N, false, false>(c->nsm, c->pg, (C *)c->d_rb, c->d_vt, T, c->d_pscr, nullptr, 0, 0, -1,
+                                               c->st);
+      }
       prof_end(c);
     }
   });
 }
-template <typename C, int N, int NS> static void launch_pencil_density_ns(amdk_ctx *c, int p0, int T, int grp, int add) {
-  const Geom &g = c->geom;
-  const size_t sm = pencil_smem<C>(N, c->pg.nz, c->ct_dens);
-  ++c->nlaunch;
-  if (grp < 0) {  // balanced schedule, -grp blocks (one batch of pairs)
-    smem_opt_in<k_pencil_density_bal<C, N, NS>>();
-    k_pencil_density_bal<C, N, NS><<<-grp, PNT, sm, c->st>>>(c->pg, plan<C>(c, 1), (const C *)c->d_rb, T, c->d_wa + p0,
-                                                             c->d_wb + p0, c->d_rhopart, c->ct_dens);
-    return;
-  }
-  const int per = (T + grp - 1) / grp;
-  smem_opt_in<k_pencil_density<C, N, NS>>();
-  k_pencil_density<C, N, NS><<<dim3(g.n1, grp), PNT, sm, c->st>>>(c->pg, plan<C>(c, 1), (const C *)c->d_rb, T, per,
-                                                                  c->d_wa + p0, c->d_wb + p0, c->d_rhopart, c->ct_dens,
-                                                                  add);
+// Density of T pairs of pg's planes: rho (=, or += with add) on pg.n1 x
+// planes, through the partial grids `part`
+template <typename C, int N, bool SEG>
+static void launch_pencil_density(int nsm, const PencilGeom &pg, const C *rb, int T, const double *wa, const double *wb,
+                                  double *part, double *rho, int add, cudaStream_t st) {
+  typedef DensShape<C, N> Sh;
+  constexpr auto K = k_pencil_density<C, N, SEG>;
+  const int nblk = (int)std::min<long>((long)pg.n1 * Sh::GA * T, (long)nsm * pencil_resident<K>(Sh::NT, Sh::smem));
+  K<<<nblk, Sh::NT, Sh::smem, st>>>(pg, pencil_tw<C, N>(), rb, T, wa, wb, part);
+  constexpr int n1f = fft_n1(N);
+  k_rho_reduce_p<<<dim3((N + 31) / 32, (pg.n1 + 31) / 32, N), dim3(32, 8), 0, st>>>(N, pg.n1, n1f, N / n1f, Sh::Z1,
+                                                                                  Sh::GA, part, rho, add, T, nblk);
 }
-template <typename C> static void launch_pencil_density(amdk_ctx *c, int p0, int T, int grp, int add) {
-  with_n(c->geom.n2, [&](auto NC) {
+// partial grids launch_pencil_density needs for nplane planes at any T: the
+// blocks that share a (plane, column group)
+template <typename C> static int density_grids(int n, int nplane, int nsm) {
+  int m = 0;
+  with_n(n, [&](auto NC) {
     constexpr int N = decltype(NC)::value;
     if constexpr (N > 0) {
-      if (c->ns_dens == 1) launch_pencil_density_ns<C, N, 1>(c, p0, T, grp, add);
-      else if (c->ns_dens == 2) launch_pencil_density_ns<C, N, 2>(c, p0, T, grp, add);
-      else launch_pencil_density_ns<C, N, 4>(c, p0, T, grp, add);
+      typedef DensShape<C, N> Sh;
+      const int nb = nsm * std::max(pencil_resident<k_pencil_density<C, N, false>>(Sh::NT, Sh::smem),
+                                    pencil_resident<k_pencil_density<C, N, true>>(Sh::NT, Sh::smem));
+      m = nb / std::max(1, nplane * Sh::GA) + 2;
     }
   });
-}
-// rho (FP64 grid) from the partial grids of a density schedule (grp > 0
-// groups per plane, grp < 0 the balanced schedule of -grp blocks over T pairs)
-static void reduce_density(amdk_ctx *c, int grp, int T, double *rho) {
-  const Geom &g = c->geom;
-  ++c->nlaunch;
-  k_rho_reduce_p<<<dim3((g.n1 + 31) / 32, (g.n1 + 31) / 32, g.n1), dim3(32, 8), 0, c->st>>>(
-      g.n1, g.n1, c->pn1, c->pn2, grp > 0 ? grp : 0, c->d_rhopart, rho, 0, grp < 0 ? T : 0, grp < 0 ? -grp : 0);
-}
-// most partial grids a plane takes under the balanced schedule of nblk blocks
-static int bal_max_slots(int n1, int T, int nblk) {
-  int m = 0;
-  for (int kx = 0; kx < n1; ++kx) m = std::max(m, bal_slots(kx, T, (long)n1 * T, nblk));
   return m;
 }
-// Pair groups of the density pencil kernel for T pairs at the current
-// precision: measured once (every candidate launched on the current buffers,
-// whose contents do not matter for the timing; the partial grids are cleared
-// before use), then cached.  Inside a graph capture the schedule model's
-// choice is used instead.
-template <typename C> static int density_groups(amdk_ctx *c, int T) {
+template <typename C> static void pencil_density(amdk_ctx *c, int p0, int T, double *rho) {
   const Geom &g = c->geom;
-  const size_t sm = pencil_smem<C>(g.n2, c->pg.nz, c->ct_dens);
-  const int key = 2 * T + (c->precision == AMDK_MIXED ? 1 : 0);
-  auto it = c->pencil_grp_cache.find(key);
-  if (it != c->pencil_grp_cache.end()) return it->second;
-  int best = pencil_density_groups(g.n1, T, c->nsm, (int)std::max<size_t>(1, (228 * 1024) / (sm + 1024)),
-                                   c->pencil_groups);
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  cudaStreamIsCapturing(c->st, &cap);
-  const std::string tkey = pencil_key(c, "pencil_density_groups_with_reduce", T) + "/ct" +
-                           std::to_string(c->ct_dens) + "/ns" + std::to_string(c->ns_dens);
-  // the balanced schedule (negative values: -blocks) for a batch that holds
-  // every pair, with at most pencil_groups partial grids per plane
-  auto bal_ok = [&](int nblk) {
-    return T == c->npairs && nblk >= 1 && (long)nblk <= (long)g.n1 * T &&
-           bal_max_slots(g.n1, T, nblk) <= c->pencil_groups;
-  };
-  int cached = 0;
-  if (cap == cudaStreamCaptureStatusNone && c->tune && tune_get(tkey, &cached) &&
-      ((cached >= 1 && cached <= std::min(c->pencil_groups, T)) || (cached < 0 && bal_ok(-cached)))) {
-    best = cached;
-  } else if (cap == cudaStreamCaptureStatusNone && c->tune) {
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
-    const long nl = c->nlaunch;
-    float best_ms = 1e30f;
-    // each candidate timed with the reduction of its partial grids: more
-    // groups spread the blocks better but leave more grids to add
-    auto run = [&](int grp) {
-      launch_pencil_density<C>(c, 0, T, grp, 0);
-      reduce_density(c, grp, T, c->d_rho);
-    };
-    // (plane, pair group) blocks, then the balanced schedule with one, two or
-    // three waves of resident blocks
-    std::vector<int> cands = {1, 2, 3, 4, 5, 6, 8, 10, 12, 16};
-    const int bps = (int)std::min<size_t>(sizeof(C) == sizeof(float2) ? 2 : 1,
-                                          std::max<size_t>(1, (228 * 1024) / (sm + 1024)));
-    for (int w = 1; w <= 3; ++w)
-      if (bal_ok(w * bps * c->nsm)) cands.push_back(-w * bps * c->nsm);
-    for (int grp : cands) {
-      if (grp > 0 && (grp > c->pencil_groups || grp > T || (grp - 1) * ((T + grp - 1) / grp) >= T))
-        continue;  // no empty group
-      run(grp);  // warm
-      float ms = 1e30f;
-      for (int rep = 0; rep < 3; ++rep) {  // the fastest of three (another context may share the GPU)
-        cudaEventRecord(e0, c->st);
-        run(grp);
-        cudaEventRecord(e1, c->st);
-        cudaEventSynchronize(e1);
-        float m1 = 0;
-        cudaEventElapsedTime(&m1, e0, e1);
-        ms = std::min(ms, m1);
-      }
-      if (ms < best_ms) {
-        best_ms = ms;
-        best = grp;
-      }
-    }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    c->nlaunch = nl;  // tuning launches are not part of the work
-    tune_put(tkey, best);
-  }
-  c->pencil_grp_cache.emplace(key, best);
-  return best;
-}
-template <typename C> static void pencil_density(amdk_ctx *c, int p0, int T) {
-  const Geom &g = c->geom;
-  const int grp = density_groups<C>(c, T);
   const double npt = (double)g.n1 * g.n2 * g.n3;
-  const int add = p0 > 0;
-  // partial grids written: groups per plane, or about one per block and plane boundary
-  const double grids = grp > 0 ? (double)grp : 1.0 + (double)(-grp) / g.n1;
-  prof_begin(c, KT_ZDENS, (double)T * rstride(c, 0) * sizeof(C) + (1.0 + add) * grids * npt * 8.0);
-  launch_pencil_density<C>(c, p0, T, grp, add);
+  prof_begin(c, KT_ZDENS, (double)T * pencil_stride(c) * sizeof(C) + npt * 8.0);
+  c->nlaunch += 2;
+  with_n(g.n2, [&](auto NC) {
+    constexpr int N = decltype(NC)::value;
+    if constexpr (N > 0)
+      launch_pencil_density<C, N, false>(c->nsm, c->pg, (const C *)c->d_rb, T, c->d_wa + p0, c->d_wb + p0, c->d_rhopart,
+                                         rho, p0 > 0, c->st);
+  });
   prof_end(c);
 }
 
@@ -818,40 +577,25 @@ template <typename C> static int density_pairs_t(amdk_ctx *c) {
   const HostSetup &h = c->hs;
   const Geom &g = c->geom;
   if (c->pencil_density) {
-    // pencil path: transposed x pass, then one block per (x-plane, pair group)
-    // the first batch stores its groups' partial grids, later batches add;
-    // groups that only later batches use are cleared first
-    const int ng_full = density_groups<C>(c, c->batch);
-    const int ng_rem = (c->npairs % c->batch) ? density_groups<C>(c, c->npairs % c->batch) : 0;
-    // the balanced schedule (ng_full < 0) runs only when one batch holds
-    // every pair: each plane's partial grids are all written, none cleared
-    const int ng = ng_full < 0 ? ng_full : std::max(ng_full, ng_rem);
-    const int ng_first = c->npairs < c->batch ? ng_rem : ng_full;
-    const size_t npt = (size_t)g.n1 * g.n2 * g.n3;
-    if (ng > ng_first)
-      CK(cudaMemsetAsync(c->d_rhopart + (size_t)ng_first * npt, 0, sizeof(double) * (ng - ng_first) * npt, c->st));
+    // pencil path: transposed x pass, then the plane kernel; later batches add to rho
     for (int p0 = 0; p0 < c->npairs; p0 += c->batch) {
       int T = std::min(c->batch, c->npairs - p0);
       xt_bwd_pair<C>(c, p0, T);
-      pencil_density<C>(c, p0, T);
+      pencil_density<C>(c, p0, T, c->d_rho);
     }
-    reduce_density(c, ng, c->npairs, c->d_rho);
     if (h.lsd) {
       // open shell: the spin-2 density from the same pair transforms, weighted
       // by the spin-2 bands only (density.f90:64-76); with all pairs in one
       // batch the ray buffer still holds them
-      if (ng > ng_first)
-        CK(cudaMemsetAsync(c->d_rhopart + (size_t)ng_first * npt, 0, sizeof(double) * (ng - ng_first) * npt, c->st));
       std::swap(c->d_wa, c->d_wa2);
       std::swap(c->d_wb, c->d_wb2);
       for (int p0 = 0; p0 < c->npairs; p0 += c->batch) {
         int T = std::min(c->batch, c->npairs - p0);
         if (c->batch < c->npairs) xt_bwd_pair<C>(c, p0, T);
-        pencil_density<C>(c, p0, T);
+        pencil_density<C>(c, p0, T, c->d_rho2);
       }
       std::swap(c->d_wa, c->d_wa2);
       std::swap(c->d_wb, c->d_wb2);
-      reduce_density(c, ng, c->npairs, c->d_rho2);
     }
   } else {
   CK(cudaMemsetAsync(c->d_rho, 0, sizeof(double) * (size_t)g.n1 * g.n2 * g.n3, c->st));
@@ -902,11 +646,12 @@ static int store_potential(amdk_ctx *c, const double2 *grid, double *vpot, void 
                        c->st));
   if (c->pencil_vpsi) {
     dim3 gt((g.n1 + 31) / 32, (g.n1 + 31) / 32, g.n1);
+    const int n1f = fft_n1(g.n1), n2f = g.n1 / n1f;
     ++c->nlaunch;
     if (c->precision == AMDK_MIXED)
-      k_v_permute<float><<<gt, dim3(32, 8), 0, c->st>>>(g.n1, g.n1, c->pn1, c->pn2, vpot, (float *)vt);
+      k_v_permute<float><<<gt, dim3(32, 8), 0, c->st>>>(g.n1, g.n1, n1f, n2f, vpot, (float *)vt);
     else
-      k_v_permute<double><<<gt, dim3(32, 8), 0, c->st>>>(g.n1, g.n1, c->pn1, c->pn2, vpot, (double *)vt);
+      k_v_permute<double><<<gt, dim3(32, 8), 0, c->st>>>(g.n1, g.n1, n1f, n2f, vpot, (double *)vt);
   }
   return 0;
 }
@@ -996,7 +741,7 @@ static bool use_slice(const amdk_ctx *c);
 // The unpack of pairs [p0, p0+T) (kinetic term, occupation scaling) fused
 // with fnonloc for the first UNPACK_NPJ projectors; further projectors are
 // added in chunks (k_fnonloc_add).  pp/pm: +G/-G positions in the ray buffer.
-template <typename C> static void unpack_h(amdk_ctx *c, int p0, int T, const int *pp, const int *pm) {
+template <typename C> static void unpack_h(amdk_ctx *c, int p0, int T, const int *pp, const int *pm, long stride) {
   typedef decltype(C().x) Rl;
   const HostSetup &h = c->hs;
   const Geom &g = c->geom;
@@ -1010,7 +755,7 @@ template <typename C> static void unpack_h(amdk_ctx *c, int p0, int T, const int
   constexpr int PAIRS = unpack_pairs<C>();
   const dim3 gu(nblk(h.ngpw, 128), (T + PAIRS - 1) / PAIRS);
   k_unpack_fnonloc<C><<<gu, 128, (size_t)2 * PAIRS * npj0 * sizeof(Rl), c->st>>>(
-      h.ngpw, c->nstate, 2 * p0, T, npj0, pp, pm, (const C *)c->d_rb, rstride(c, 0), scale, c->d_hg, h.tpiba2,
+      h.ngpw, c->nstate, 2 * p0, T, npj0, pp, pm, (const C *)c->d_rb, stride, scale, c->d_hg, h.tpiba2,
       c->d_occ, c->d_P, c->d_D, c->nproj, c->d_c0, c->d_c2, c->nproj > npj0 ? nullptr : bmax, 0);
   // with projector chunks still to add, C2 is sliced from scratch
   c->c2max_ok = bmax != nullptr && c->nproj <= npj0;
@@ -1034,7 +779,7 @@ template <typename C> static int apply_h_t(amdk_ctx *c) {
       xt_bwd_pair<C>(c, p0, T);
       pencil_vpsi<C>(c, T, p0);
       xt_fwd<C>(c, T);
-      unpack_h<C>(c, p0, T, c->d_postp, c->d_postm);
+      unpack_h<C>(c, p0, T, c->d_postp, c->d_postm, pencil_stride(c));
     }
     CK(cudaGetLastError());
     return 0;
@@ -1053,7 +798,7 @@ template <typename C> static int apply_h_t(amdk_ctx *c) {
     z_pass<C, Z_VPSI>(c, 0, T, nullptr, nullptr);
     y_pass<C>(c, 0, -1, T);
     x_fwd<C>(c, 0, T);
-    unpack_h<C>(c, p0, T, c->d_posp, c->d_posm);
+    unpack_h<C>(c, p0, T, c->d_posp, c->d_posm, rstride(c, 0));
   }
   CK(cudaGetLastError());
   return 0;
@@ -1604,9 +1349,6 @@ static void set_pair_precision(amdk_ctx *c, int prec) {
   c->precision = prec;
   c->pencil_vpsi = c->pv_p[q];
   c->pencil_density = c->pd_p[q];
-  c->ct_vpsi = c->ctv_p[q];
-  c->ct_dens = c->ctd_p[q];
-  c->ns_dens = c->nsd_p[q];
 }
 
 // Ray coordinates (ky, kz) of the density-sphere x-rays in the reference's
@@ -1636,6 +1378,29 @@ static void ray_tables(const HostSetup &h, std::vector<int> &ray_ky, std::vector
     int kxp = ((ix % n1) + n1) % n1, kxm = ((-ix % n1) + n1) % n1;
     posp[ig] = rp * n1 + kxp;
     posm[ig] = rm * n1 + kxm;
+  }
+}
+
+// The pencil path's rays: ky by ky, the kz of each consecutive (signed order),
+// so that a ky's rays are one interval of the buffer; a gap in an interval
+// (skewed cells can have one) is filled with a ray that carries no G vector
+// (-1).  rays[j]: the ray in the reference's numbering; cols[ky]: ray_pack.
+static void pencil_rays(int n, const std::vector<int> &ray_ky, const std::vector<int> &ray_kz, int nrays,
+                        std::vector<int> &rays, std::vector<int> &cols) {
+  std::vector<int> at((size_t)n * n, -1);
+  for (int r = 0; r < nrays; r++) at[(size_t)ray_ky[r] * n + ray_kz[r]] = r;
+  rays.clear();
+  cols.assign(n, ray_pack(0, 1, -1));
+  for (int ky = 0; ky < n; ky++) {
+    int lo = n, hi = -n;
+    for (int k = -(n / 2); k < (n + 1) / 2; k++)
+      if (at[(size_t)ky * n + (k + n) % n] >= 0) {
+        lo = std::min(lo, k);
+        hi = k;
+      }
+    if (lo > hi) continue;
+    cols[ky] = ray_pack((int)rays.size() - lo, lo, hi);
+    for (int k = lo; k <= hi; k++) rays.push_back(at[(size_t)ky * n + (k + n) % n]);
   }
 }
 
@@ -1722,8 +1487,6 @@ static int build_device(amdk_ctx *c) {
     RC(c->alloc(&c->d_part2, (size_t)RED_BLOCKS * 4));
     const char *env = getenv("AMDK_NO_GRAPHS");
     c->use_graphs = !(env && env[0] == '1');
-    const char *nt = getenv("AMDK_NO_TUNE");
-    c->tune = !(nt && nt[0] == '1');
     const char *no = getenv("AMDK_NO_OVERLAP");
     c->overlap = !(no && no[0] == '1');
   }
@@ -1778,37 +1541,20 @@ static int build_device(amdk_ctx *c) {
   c->h_info[0] = c->h_info[1] = 0;
   CK(cudaMemset(c->d_scal, 0, S_NSCAL * sizeof(double)));
   // Pencil path for the pair transforms (cubic grids with a specialised
-  // length whose slab plane fits in shared memory): V(r)psi and the density
-  // go plane by plane through shared memory with no slab buffer in HBM.
-  // Decided for both pair precisions (index 0 FP64, 1 mixed) so that
-  // amdk_set_precision can switch between them; buffers are sized for FP64.
+  // length): V(r)psi and the density go plane by plane through shared memory
+  // with no slab buffer in HBM.  Its kernels hold a slab of (n-1)/4 planes on
+  // each side of kz = 0 and the same range of ky: the sphere of a grid that
+  // also holds the density sphere (checked).
   {
     bool known = false;
     with_n(n1, [&](auto NC) { known = decltype(NC)::value > 0; });
-    const bool ok = (n1 == n2 && n2 == n3) && known && g.nz[0] < 255;  // slab planes fit the packed table
-    const size_t lim = 227 * 1024;
-    const int nz0 = g.nz[0];
+    bool ok = n1 == n2 && n2 == n3 && known;
+    const int hmax = (n1 - 1) / 4;
+    for (int r = 0; r < h.ngrays && ok; r++)
+      ok = std::min(ray_ky[r], n2 - ray_ky[r]) <= hmax && std::min(ray_kz[r], n3 - ray_kz[r]) <= hmax;
     const char *env = getenv("AMDK_NO_PENCIL");
     const bool off = env && env[0] == '1';
-    if (ok) {
-      c->pn1 = fft_n1(n1);
-      c->pn2 = n1 / c->pn1;
-      // V(r)psi: two blocks per SM when the tile can stay at least half the
-      // plane wide, else one
-      int ct2 = pencil_tile<double2>(n1, nz0, 0, lim / 2), ct1 = pencil_tile<double2>(n1, nz0, 0, lim);
-      c->ctv_p[0] = (2 * ct2 >= n1) ? ct2 : ct1;
-      ct2 = pencil_tile<float2>(n1, nz0, 0, lim / 2);
-      ct1 = pencil_tile<float2>(n1, nz0, 0, lim);
-      c->ctv_p[1] = (2 * ct2 >= n1) ? ct2 : ct1;
-      // density: equal column tiles (1, 2 or 4) whose sums fit 1, 2 or 4
-      // register slots; two blocks per SM when possible
-      density_tiles(n1, nz0, sizeof(double2), lim, &c->ctd_p[0], &c->nsd_p[0]);
-      density_tiles(n1, nz0, sizeof(float2), lim, &c->ctd_p[1], &c->nsd_p[1]);
-    }
-    for (int q = 0; q < 2; ++q) {
-      c->pv_p[q] = ok && !off && c->ctv_p[q] >= 8;
-      c->pd_p[q] = ok && !off && c->ctd_p[q] >= 8;
-    }
+    for (int q = 0; q < 2; ++q) c->pv_p[q] = c->pd_p[q] = ok && !off;
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -1829,7 +1575,9 @@ static int build_device(amdk_ctx *c) {
   // pair batch: all pairs at once on the pencil path, else 8
   if (c->batch <= 0) c->batch = pencil_all ? c->npairs : 8;
   c->batch = std::max(1, std::min(c->batch, c->npairs));
-  size_t rb = (size_t)c->batch * rstride(c, 0) * sizeof(double2);
+  std::vector<int> prays, pcols;  // pencil path: its rays (of the reference's numbering) and table
+  if (c->pv_p[0] || c->pv_p[1]) pencil_rays(n1, ray_ky, ray_kz, h.ngrays, prays, pcols);
+  size_t rb = (size_t)c->batch * std::max<long>(rstride(c, 0), (long)prays.size() * n1) * sizeof(double2);
   const size_t rbf = 2 * (size_t)rstride(c, 1) * sizeof(double2);
   size_t sb = 2 * (size_t)sstride(c, 1) * sizeof(double2);
   if (!(c->pv_p[0] && c->pd_p[0] && c->pv_p[1] && c->pd_p[1]))
@@ -1840,26 +1588,31 @@ static int build_device(amdk_ctx *c) {
   c->fftbuf_bytes = rb + rbf + sb;
   set_pair_precision(c, c->precision);
   if (c->pv_p[0] || c->pv_p[1] || c->pd_p[0] || c->pd_p[1]) {
-    std::vector<int> rpos(h.ngrays), zinv(n3, -1), zl0(g.nz[0]), postp(h.ngpw), postm(h.ngpw);
-    CK(cudaMemcpy(zl0.data(), c->d_zlist[0], sizeof(int) * g.nz[0], cudaMemcpyDeviceToHost));
-    for (int zi = 0; zi < g.nz[0]; zi++) zinv[zl0[zi]] = zi;
-    for (int r = 0; r < h.ngrays; r++) rpos[r] = zinv[ray_kz[r]] * (n2 + 1) + ray_ky[r];
+    const int R = (int)prays.size();
+    std::vector<int> pidx(h.ngrays), postp(h.ngpw), postm(h.ngpw);
+    for (int j = 0; j < R; j++)
+      if (prays[j] >= 0) pidx[prays[j]] = j;
     // G -> transposed ray buffer position kx*R + ray
     for (int ig = 0; ig < h.ngpw; ig++) {
-      postp[ig] = (posp[ig] % n1) * h.ngrays + posp[ig] / n1;
-      postm[ig] = (posm[ig] % n1) * h.ngrays + posm[ig] / n1;
+      postp[ig] = (posp[ig] % n1) * R + pidx[posp[ig] / n1];
+      postm[ig] = (posm[ig] % n1) * R + pidx[posm[ig] / n1];
     }
-    RC(c->up(&c->d_rpos, rpos));
-    RC(c->up(&c->d_zinv, zinv));
+    RC(c->up(&c->d_cols, pcols));
     RC(c->up(&c->d_postp, postp));
     RC(c->up(&c->d_postm, postm));
-    std::vector<int> gmapt((size_t)n1 * h.ngrays);
-    for (int r = 0; r < h.ngrays; r++)
-      for (int k = 0; k < n1; k++) gmapt[(size_t)k * h.ngrays + r] = gmap[(size_t)r * n1 + k];
+    std::vector<int> gmapt((size_t)n1 * R, 0);
+    for (int j = 0; j < R; j++)
+      if (prays[j] >= 0)
+        for (int k = 0; k < n1; k++) gmapt[(size_t)k * R + j] = gmap[(size_t)prays[j] * n1 + k];
     RC(c->up(&c->d_gmapt, gmapt));
-    c->pg = pencil_geom_1gpu(n1, n2, n3, h.ngrays, g.nz[0], c->d_rpos, c->d_zinv, c->d_zlist[0], c->d_gmapt);
-    c->pencil_groups = std::max(1, std::min(c->batch, 16));
-    if (c->pd_p[0] || c->pd_p[1]) RC(c->alloc(&c->d_rhopart, (size_t)c->pencil_groups * npt));
+    c->pg = pencil_geom_1gpu(n1, n2, n3, R, c->d_cols, c->d_gmapt);
+    const int grids = std::max(density_grids<double2>(n1, n1, c->nsm), density_grids<float2>(n1, n1, c->nsm));
+    RC(c->alloc(&c->d_rhopart, (size_t)grids * npt));
+    if (const size_t sb2 = std::max(vpsi_scratch_bytes<double2>(n1, c->nsm), vpsi_scratch_bytes<float2>(n1, c->nsm))) {
+      char *scr;
+      RC(c->alloc(&scr, sb2));
+      c->d_pscr = scr;
+    }
     if (c->pv_p[0] || c->pv_p[1]) {
       char *vt;
       RC(c->alloc(&vt, (size_t)npt * sizeof(double)));
@@ -2029,7 +1782,7 @@ template <typename C> static int seg_a_overlap(amdk_ctx *c) {
   CK(cudaMemcpyAsync(c->h_pin, c->d_scal, sizeof(double) * S_NSCAL, cudaMemcpyDeviceToHost, c->st));
   pencil_vpsi<C>(c, T);
   xt_fwd<C>(c, T);
-  unpack_h<C>(c, 0, T, c->d_postp, c->d_postm);
+  unpack_h<C>(c, 0, T, c->d_postp, c->d_postm, pencil_stride(c));
   RC(do_gradient(c));
   CK(cudaMemcpyAsync(c->h_pin + S_NSCAL, c->d_scal + S_GMAX, sizeof(double), cudaMemcpyDeviceToHost, c->st));
   return 0;
@@ -2200,8 +1953,8 @@ static int slab_partition(const HostSetup &h, int nranks, const std::vector<int>
                           const std::vector<int> &ray_kz, const std::vector<int> &posp, std::vector<int> &ray_owner,
                           std::vector<int> &plane0) {
   const int n1 = h.nr[0], n2 = h.nr[1], n3 = h.nr[2], R = h.ngrays;
-  if (nranks < 1 || nranks > PG_MAXSEG || nranks > n1) {
-    set_error("slab decomposition: nranks must be 1.." + std::to_string(std::min(PG_MAXSEG, n1)));
+  if (nranks < 1 || nranks > AMDK_SLAB_MAXRANKS || nranks > n1) {
+    set_error("slab decomposition: nranks must be 1.." + std::to_string(std::min(AMDK_SLAB_MAXRANKS, n1)));
     return AMDK_ERR_BADARG;
   }
   std::vector<long> ng(R, 0);
@@ -2248,13 +2001,14 @@ struct amdk_slab {
   int ng = 0, nray_loc = 0, gzero = -1, nplane = 0, nray = 0;
   std::vector<int> plane0, seg_r0, local_g;
   // sender side: local G code of (kx, local ray), planes and local rays of
-  // each local G's +G / -G position, |G|^2; receiver side: rpos of every ray
-  // in owner order
+  // each local G's +G / -G position, |G|^2; receiver side: the place of every
+  // (ky, slab row)'s ray in the source segments
   int *d_gmapt = nullptr, *d_kxp = nullptr, *d_rlp = nullptr, *d_kxm = nullptr, *d_rlm = nullptr;
-  int *d_pp = nullptr, *d_pm = nullptr, *d_rpos = nullptr;
+  int *d_pp = nullptr, *d_pm = nullptr;
+  int2 *d_seg = nullptr;
   double *d_hg = nullptr, *d_rhopart = nullptr;
-  void *d_vp = nullptr;
-  int pos_T = -1, groups_max = 8;
+  void *d_vp = nullptr, *d_pscr = nullptr;
+  int pos_T = -1;
   std::vector<void *> allocs;
   template <typename T> int alloc(T **p, size_t n) {
     RC(dalloc(p, n));
@@ -2311,12 +2065,15 @@ static int slab_create(amdk_ctx *c, int nranks, int rank, amdk_slab *s) {
   }
   s->seg_r0[nranks] = (int)order.size();
   s->nray_loc = s->seg_r0[rank + 1] - s->seg_r0[rank];
-  // the ray's plane position, as in the one-GPU pencil tables
-  std::vector<int> zl0(c->geom.nz[0]), zinv(h.nr[2], -1), rpos(h.ngrays);
-  CK(cudaMemcpy(zl0.data(), c->d_zlist[0], sizeof(int) * zl0.size(), cudaMemcpyDeviceToHost));
-  for (int zi = 0; zi < (int)zl0.size(); zi++) zinv[zl0[zi]] = zi;
-  for (int j = 0; j < h.ngrays; j++) rpos[j] = zinv[ray_kz[order[j]]] * (n2 + 1) + ray_ky[order[j]];
-  RC(s->up(&s->d_rpos, rpos));
+  // {first ray, place | rays << 16} of the source segment holding the ray at
+  // (ky, slab row zi: kz = zi or zi - nz)
+  const int hz = (n1 - 1) / 4, nz = 2 * hz + 1;
+  std::vector<int2> seg((size_t)n2 * nz, make_int2(0, 0));
+  for (int r = 0; r < h.ngrays; r++) {
+    const int o = owner[r], zi = ray_kz[r] <= hz ? ray_kz[r] : ray_kz[r] - n2 + nz;
+    seg[(size_t)ray_ky[r] * nz + zi] = make_int2(s->seg_r0[o], rloc[r] | (s->seg_r0[o + 1] - s->seg_r0[o]) << 16);
+  }
+  RC(s->up(&s->d_seg, seg));
   // local G vectors (increasing global index) and their tables
   const int R = s->nray_loc;
   std::vector<int> gmapt((size_t)n1 * std::max(R, 1), 0), kxp, rlp, kxm, rlm;
@@ -2345,7 +2102,13 @@ static int slab_create(amdk_ctx *c, int nranks, int rank, amdk_slab *s) {
   RC(s->alloc(&s->d_pp, std::max(s->ng, 1)));
   RC(s->alloc(&s->d_pm, std::max(s->ng, 1)));
   const size_t pl = (size_t)s->nplane * n1 * n1;  // cubic grid (pencil path)
-  RC(s->alloc(&s->d_rhopart, (size_t)s->groups_max * pl));
+  const int grids = q ? density_grids<float2>(n1, s->nplane, c->nsm) : density_grids<double2>(n1, s->nplane, c->nsm);
+  RC(s->alloc(&s->d_rhopart, (size_t)grids * pl));
+  if (const size_t sb = q ? vpsi_scratch_bytes<float2>(n1, c->nsm) : vpsi_scratch_bytes<double2>(n1, c->nsm)) {
+    char *scr;
+    RC(s->alloc(&scr, sb));
+    s->d_pscr = scr;
+  }
   char *vp;
   RC(s->alloc(&vp, pl * sizeof(double)));
   s->d_vp = vp;
@@ -2370,8 +2133,7 @@ static int slab_check_pairs(const amdk_slab *s, int band0, int npairs) {
 // sender side: local rays, layout [kx][t][ray] (rank-major send order)
 static PencilGeom slab_xgeom(const amdk_slab *s, int T) {
   const HostSetup &h = s->c->hs;
-  PencilGeom g = pencil_geom_1gpu(h.nr[0], h.nr[1], h.nr[2], s->nray_loc, s->c->geom.nz[0], nullptr, nullptr, nullptr,
-                                  s->d_gmapt);
+  PencilGeom g = pencil_geom_1gpu(h.nr[0], h.nr[1], h.nr[2], s->nray_loc, nullptr, s->d_gmapt);
   g.xt_t = s->nray_loc;
   g.xt_x = (long)T * s->nray_loc;
   return g;
@@ -2379,13 +2141,11 @@ static PencilGeom slab_xgeom(const amdk_slab *s, int T) {
 // receiver side: this rank's planes, every ray, one segment per source rank
 static PencilGeom slab_pgeom(const amdk_slab *s, int T) {
   const HostSetup &h = s->c->hs;
-  PencilGeom g = pencil_geom_1gpu(s->nplane, h.nr[1], h.nr[2], s->nray, s->c->geom.nz[0], s->d_rpos, s->c->d_zinv,
-                                  s->c->d_zlist[0], nullptr);
+  PencilGeom g = pencil_geom_1gpu(s->nplane, h.nr[1], h.nr[2], s->nray, nullptr, nullptr);
+  g.seg = s->d_seg;
   g.pr_t = 1;
   g.pr_x = T;
-  g.nseg = s->nranks;
   g.seg_mul = (long)s->nplane * T;
-  for (int o = 0; o <= s->nranks; o++) g.seg_r0[o] = s->seg_r0[o];
   return g;
 }
 
@@ -2411,54 +2171,32 @@ static int slab_pairs_out_t(amdk_slab *s, const double2 *c0, int band0, int T, C
 template <typename C> static int slab_vpsi_t(amdk_slab *s, C *recv, int T, const double *v, cudaStream_t st) {
   typedef decltype(C().x) Rl;
   amdk_ctx *c = s->c;
-  const int n = c->hs.nr[1], q = (s->precision == AMDK_MIXED) ? 1 : 0;
-  ++c->nlaunch;
-  k_v_permute<Rl><<<dim3((s->nplane + 31) / 32, (n + 31) / 32, n), dim3(32, 8), 0, st>>>(n, s->nplane, c->pn1, c->pn2,
-                                                                                      v, (Rl *)s->d_vp);
+  const int n = c->hs.nr[1], n1f = fft_n1(n);
+  if (s->nplane == 0) return 0;
+  c->nlaunch += 2;
+  k_v_permute<Rl><<<dim3((s->nplane + 31) / 32, (n + 31) / 32, n), dim3(32, 8), 0, st>>>(n, s->nplane, n1f, n / n1f, v,
+                                                                                      (Rl *)s->d_vp);
   const PencilGeom gp = slab_pgeom(s, T);
-  const int ct = c->ctv_p[q];
   with_n(n, [&](auto NC) {
     constexpr int N = decltype(NC)::value;
-    if constexpr (N > 0) {
-      smem_opt_in<k_pencil_vpsi<C, N>>();
-      ++c->nlaunch;
-      k_pencil_vpsi<C, N><<<dim3(s->nplane, T), PNT, pencil_smem<C>(N, gp.nz, ct), st>>>(
-          gp, plan<C>(c, 1), recv, (const Rl *)s->d_vp, ct, nullptr, 0, 0, -1);
-    }
+    if constexpr (N > 0)
+      launch_pencil_vpsi<C, N, true, false>(c->nsm, gp, recv, s->d_vp, T, s->d_pscr, nullptr, 0, 0, -1, st);
   });
   CK(cudaGetLastError());
   return 0;
 }
-template <typename C, int N, int NS>
-static void slab_density_launch(amdk_slab *s, const C *recv, int band0, int T, int grp, int ct, cudaStream_t st) {
-  amdk_ctx *c = s->c;
-  const PencilGeom gp = slab_pgeom(s, T);
-  const int per = (T + grp - 1) / grp;
-  smem_opt_in<k_pencil_density<C, N, NS>>();
-  ++c->nlaunch;
-  k_pencil_density<C, N, NS><<<dim3(s->nplane, grp), PNT, pencil_smem<C>(N, gp.nz, ct), st>>>(
-      gp, plan<C>(c, 1), recv, T, per, c->d_wa + band0 / 2, c->d_wb + band0 / 2, s->d_rhopart, ct, 0);
-}
 template <typename C>
 static int slab_density_t(amdk_slab *s, const C *recv, int band0, int T, double *rho, int add, cudaStream_t st) {
   amdk_ctx *c = s->c;
-  const int n = c->hs.nr[1], q = (s->precision == AMDK_MIXED) ? 1 : 0;
-  const int ct = c->ctd_p[q], ns = c->nsd_p[q];
-  // pair groups: enough blocks for two waves, at most groups_max grids
-  int grp = std::max(1, std::min({T, s->groups_max, (2 * c->nsm + s->nplane - 1) / s->nplane}));
-  const int per = (T + grp - 1) / grp;
-  grp = (T + per - 1) / per;  // no empty group
-  with_n(n, [&](auto NC) {
+  if (s->nplane == 0) return 0;
+  c->nlaunch += 2;
+  const PencilGeom gp = slab_pgeom(s, T);
+  with_n(c->hs.nr[1], [&](auto NC) {
     constexpr int N = decltype(NC)::value;
-    if constexpr (N > 0) {
-      if (ns == 1) slab_density_launch<C, N, 1>(s, recv, band0, T, grp, ct, st);
-      else if (ns == 2) slab_density_launch<C, N, 2>(s, recv, band0, T, grp, ct, st);
-      else slab_density_launch<C, N, 4>(s, recv, band0, T, grp, ct, st);
-    }
+    if constexpr (N > 0)
+      launch_pencil_density<C, N, true>(c->nsm, gp, recv, T, c->d_wa + band0 / 2, c->d_wb + band0 / 2, s->d_rhopart, rho,
+                                        add, st);
   });
-  ++c->nlaunch;
-  k_rho_reduce_p<<<dim3((n + 31) / 32, (s->nplane + 31) / 32, n), dim3(32, 8), 0, st>>>(
-      n, s->nplane, c->pn1, c->pn2, grp, s->d_rhopart, rho, add, 0, 0);
   CK(cudaGetLastError());
   return 0;
 }

@@ -107,42 +107,74 @@ template <typename C> struct Plan {
   const C *w;   // w[k] = exp(-2 pi i k/n), k < n (device)
 };
 
-// Radix-r DFT with exponent sign sg: y_p = sum_q a_q exp(sg 2 pi i p q / r)
-template <typename C> __device__ __forceinline__ void dft_r(C *a, int r, int sg) {
+// a + i sg b and its scaled form a + i sg s b: the quarter turn is folded into
+// the two scalar additions (FMAs) instead of forming i b
+template <typename C> __device__ __forceinline__ C caddi(C a, C b, int sg) {
+  C r;
+  r.x = sg > 0 ? a.x - b.y : a.x + b.y;
+  r.y = sg > 0 ? a.y + b.x : a.y - b.x;
+  return r;
+}
+template <typename C, typename R> __device__ __forceinline__ C cfmai(C a, R s, C b) {  // a + i s b
+  C r;
+  r.x = a.x - s * b.y;
+  r.y = a.y + s * b.x;
+  return r;
+}
+template <typename C> __device__ __forceinline__ C cneg(C a) {
+  a.x = -a.x;
+  a.y = -a.y;
+  return a;
+}
+// x + y and x - y where zx / zy say (at compile time, after unrolling) that a term is zero
+template <typename C> __device__ __forceinline__ C addz(C x, bool zx, C y, bool zy) {
+  return zx ? y : (zy ? x : cadd(x, y));
+}
+template <typename C> __device__ __forceinline__ C subz(C x, bool zx, C y, bool zy) {
+  return zy ? x : (zx ? cneg(y) : csub(x, y));
+}
+// radix-r DFT as dft_r with z[q] set where input q is known to be zero
+template <typename C> __device__ __forceinline__ void dft_rz(C *a, const bool *z, int r, int sg) {
   typedef decltype(a[0].x) R;
   if (r == 2) {
-    C t = a[0];
-    a[0] = cadd(t, a[1]);
-    a[1] = csub(t, a[1]);
+    const C t = a[0];
+    a[0] = addz(t, z[0], a[1], z[1]);
+    a[1] = subz(t, z[0], a[1], z[1]);
   } else if (r == 4) {
-    C t0 = cadd(a[0], a[2]), t1 = csub(a[0], a[2]);
-    C t2 = cadd(a[1], a[3]), t3 = cimul(csub(a[1], a[3]), sg);
-    a[0] = cadd(t0, t2);
-    a[2] = csub(t0, t2);
-    a[1] = cadd(t1, t3);
-    a[3] = csub(t1, t3);
+    const bool z02 = z[0] && z[2], z13 = z[1] && z[3];
+    const C t0 = addz(a[0], z[0], a[2], z[2]), t1 = subz(a[0], z[0], a[2], z[2]);
+    const C t2 = addz(a[1], z[1], a[3], z[3]), t3 = subz(a[1], z[1], a[3], z[3]);
+    a[0] = addz(t0, z02, t2, z13);
+    a[2] = subz(t0, z02, t2, z13);
+    a[1] = z13 ? t1 : (z02 ? cimul(t3, sg) : caddi(t1, t3, sg));
+    a[3] = z13 ? t1 : (z02 ? cimul(t3, -sg) : caddi(t1, t3, -sg));
   } else if (r == 3) {
-    const R c3 = (R)-0.5, s3 = (R)0.86602540378443864676;
-    C t1 = cadd(a[1], a[2]), t2 = cimul(cscale(csub(a[1], a[2]), s3), sg);
-    C m = cfmas(t1, c3, a[0]);
-    a[0] = cadd(a[0], t1);
-    a[1] = cadd(m, t2);
-    a[2] = csub(m, t2);
-  } else {  // r == 5
+    const R s3 = (R)0.86602540378443864676 * (R)sg;
+    const C t1 = addz(a[1], z[1], a[2], z[2]), d = subz(a[1], z[1], a[2], z[2]);
+    const C m = z[0] ? cscale(t1, (R)-0.5) : cfmas(t1, (R)-0.5, a[0]);
+    a[0] = addz(a[0], z[0], t1, z[1] && z[2]);
+    a[1] = cfmai(m, s3, d);
+    a[2] = cfmai(m, -s3, d);
+  } else {  // r == 5 (no zero inputs: it is never a first stage)
     const R c1 = (R)0.30901699437494742410, c2 = (R)-0.80901699437494742410;
     const R s1 = (R)0.95105651629515357212, s2 = (R)0.58778525229247312917;
-    C t1 = cadd(a[1], a[4]), t2 = cadd(a[2], a[3]);
-    C t3 = csub(a[1], a[4]), t4 = csub(a[2], a[3]);
-    C m1 = cfmas(t2, c2, cfmas(t1, c1, a[0]));
-    C m2 = cfmas(t2, c1, cfmas(t1, c2, a[0]));
-    C n1 = cimul(cfmas(t4, s2, cscale(t3, s1)), sg);
-    C n2 = cimul(cfmas(t4, -s1, cscale(t3, s2)), sg);
+    const C t1 = cadd(a[1], a[4]), t2 = cadd(a[2], a[3]);
+    const C t3 = csub(a[1], a[4]), t4 = csub(a[2], a[3]);
+    const C m1 = cfmas(t2, c2, cfmas(t1, c1, a[0]));
+    const C m2 = cfmas(t2, c1, cfmas(t1, c2, a[0]));
+    const C n1 = cfmas(t4, s2, cscale(t3, s1));
+    const C n2 = cfmas(t4, -s1, cscale(t3, s2));
     a[0] = cadd(a[0], cadd(t1, t2));
-    a[1] = cadd(m1, n1);
-    a[4] = csub(m1, n1);
-    a[2] = cadd(m2, n2);
-    a[3] = csub(m2, n2);
+    a[1] = caddi(m1, n1, sg);
+    a[4] = caddi(m1, n1, -sg);
+    a[2] = caddi(m2, n2, sg);
+    a[3] = caddi(m2, n2, -sg);
   }
+}
+// y_p = sum_q a_q exp(sg 2 pi i p q / r)
+template <typename C> __device__ __forceinline__ void dft_r(C *a, int r, int sg) {
+  const bool z[5] = {false, false, false, false, false};
+  dft_rz(a, z, r, sg);
 }
 
 // Stockham FFT of L lines held in shared memory, element k of line l at
@@ -209,43 +241,105 @@ __host__ __device__ constexpr int fft_n1(int n) {
   return best;
 }
 
-// y_k = sum_j v_j exp(SG 2 pi i jk/R), natural order in and out
+// a W_R^(T m), W_R = exp(-2 pi i / R), for an m known after unrolling:
+// quarter turns cost no multiplication
+template <typename C, int R, int T> __device__ __forceinline__ C ctw_mul(C a, int m) {
+  m %= R;
+  if (m == 0) return a;
+  if (2 * m == R) return cneg(a);
+  if (4 * m == R) return cimul(a, -T);
+  if (4 * m == 3 * R) return cimul(a, T);
+  C w = ctw<C>(ctw_off(R) + m);
+  if (T < 0) w.y = -w.y;
+  return cmul(a, w);
+}
+
+__host__ __device__ constexpr int dft_gcd(int a, int b) { return b == 0 ? a : dft_gcd(b, a % b); }
+// the e < A*B with e = 1 mod A and e = 0 mod B (A, B coprime)
+__host__ __device__ constexpr int crt_unit(int A, int B) {
+  for (int e = 0; e < A * B; e += B)
+    if (e % A == 1 % A) return e;
+  return 0;
+}
+
+// y_k = sum_j v_j exp(SG 2 pi i jk/R), natural order in and out.  R > 5 is
+// A x B; coprime factors (6, 10, 12) are indexed as Good (1958) and Thomas
+// (1963) do, which needs no twiddles between the stages.
+//   run       every input and output
+//   run_in    inputs LO <= j < HI are zero (and not read): radix A first, on
+//             inputs B apart, so that most of its terms are copies
+//   run_out   radix A last: outputs the caller does not use cost nothing (the
+//             unused half of the last butterflies is dead code); only inputs
+//             j = GR (mod GA) are read, the others are zero (GA divides A)
 template <typename C, int R, int SG> struct Dft {
-  static __device__ __forceinline__ void run(C (&v)[R]) {
-    if constexpr (R == 2 || R == 3 || R == 4 || R == 5) {
-      dft_r(v, R, SG);
-    } else if constexpr (R > 5) {
-      constexpr int A = reg_radix(R), B = R / A;
-      // j = j2 + B*j1: DFT_A over j1, twiddle W_R^(j2 k1), DFT_B over j2
+  static constexpr int A = R <= 5 ? 1 : reg_radix(R), B = R <= 5 ? R : R / A;
+  static constexpr bool PFA = R > 5 && dft_gcd(A, B) == 1;
+  template <int LO, int HI> static __device__ __forceinline__ void run_in(C (&v)[R]) {
+    if constexpr (R <= 5) {
+      bool z[R];
 #pragma unroll
-      for (int j2 = 0; j2 < B; ++j2) {
+      for (int j = 0; j < R; ++j) z[j] = false;
+      dft_rz(v, z, R, SG);
+    } else {
+      constexpr int eA = crt_unit(A, B), eB = crt_unit(B, A);
+      C t[R];  // t[b + B*ka]
+#pragma unroll
+      for (int b = 0; b < B; ++b) {
         C a[A];
+        bool z[A];
 #pragma unroll
-        for (int j1 = 0; j1 < A; ++j1) a[j1] = v[j2 + B * j1];
-        Dft<C, A, SG>::run(a);
-#pragma unroll
-        for (int k1 = 0; k1 < A; ++k1) {
-          if ((j2 * k1) % R == 0) {
-            v[j2 + B * k1] = a[k1];
-          } else {
-            C w = ctw<C>(ctw_off(R) + (j2 * k1) % R);
-            if (SG > 0) w.y = -w.y;
-            v[j2 + B * k1] = cmul(a[k1], w);
-          }
+        for (int i = 0; i < A; ++i) {
+          const int j = PFA ? (B * i + A * b) % R : b + B * i;
+          a[i] = v[j];
+          z[i] = j >= LO && j < HI;
         }
-      }
-      C o[R];
+        dft_rz(a, z, A, SG);
 #pragma unroll
-      for (int k1 = 0; k1 < A; ++k1) {
-        C b[B];
-#pragma unroll
-        for (int j2 = 0; j2 < B; ++j2) b[j2] = v[j2 + B * k1];
-        Dft<C, B, SG>::run(b);
-#pragma unroll
-        for (int k2 = 0; k2 < B; ++k2) o[k1 + A * k2] = b[k2];
+        for (int ka = 0; ka < A; ++ka) t[b + B * ka] = PFA ? a[ka] : ctw_mul<C, R, -SG>(a[ka], b * ka);
       }
 #pragma unroll
-      for (int k = 0; k < R; ++k) v[k] = o[k];
+      for (int ka = 0; ka < A; ++ka) {
+        C u[B];
+#pragma unroll
+        for (int b = 0; b < B; ++b) u[b] = t[b + B * ka];
+        Dft<C, B, SG>::run(u);
+#pragma unroll
+        for (int kb = 0; kb < B; ++kb) v[PFA ? (ka * eA + kb * eB) % R : ka + A * kb] = u[kb];
+      }
+    }
+  }
+  static __device__ __forceinline__ void run(C (&v)[R]) { run_in<R, R>(v); }
+  template <int GA, int GR> static __device__ __forceinline__ void run_out(C (&v)[R]) {
+    if constexpr (R <= 5) {
+      run(v);
+    } else {
+      constexpr int eA = crt_unit(A, B), eB = crt_unit(B, A);
+      C t[R];  // t[kb + B*i]
+#pragma unroll
+      for (int i = 0; i < A; ++i) {
+        // the inputs of sub-transform i are all = i (mod GA) (GA divides A), up
+        // to the unit B of the coprime index map
+        if ((PFA ? B * i : i) % GA != GR) continue;
+        C u[B];
+#pragma unroll
+        for (int b = 0; b < B; ++b) u[b] = v[PFA ? (B * i + A * b) % R : i + A * b];
+        Dft<C, B, SG>::run(u);
+#pragma unroll
+        for (int kb = 0; kb < B; ++kb) t[kb + B * i] = PFA ? u[kb] : ctw_mul<C, R, -SG>(u[kb], i * kb);
+      }
+#pragma unroll
+      for (int kb = 0; kb < B; ++kb) {
+        C a[A];
+        bool z[A];
+#pragma unroll
+        for (int i = 0; i < A; ++i) {
+          z[i] = (PFA ? B * i : i) % GA != GR;
+          if (!z[i]) a[i] = t[kb + B * i];
+        }
+        dft_rz(a, z, A, SG);
+#pragma unroll
+        for (int ka = 0; ka < A; ++ka) v[PFA ? (ka * eA + kb * eB) % R : kb + B * ka] = a[ka];
+      }
     }
   }
 };
