@@ -8,6 +8,7 @@
 #include <cstring>
 #include <functional>
 #include <map>
+#include <numeric>
 #include <mutex>
 #include <type_traits>
 #include <string>
@@ -100,6 +101,7 @@ struct amdk_ctx {
   // FP64 tensor-core GEMMs: split-K partial tiles (one buffer per stream)
   // and the poll limit of their pipeline waits (options.reserved[1])
   double *d_dgpart = nullptr, *d_dgpart2 = nullptr;
+  double *d_gpad = nullptr;  // a band-space matrix with an odd leading dimension, padded
   long dg_plim = SG_SPIN;
   cudaEvent_t ev_fork = nullptr, ev_side_done = nullptr;
   size_t fftbuf_bytes = 0;
@@ -112,6 +114,7 @@ struct amdk_ctx {
   // projectors (compact list)
   int nproj = 0;
   std::vector<int> p_isa, p_is, p_iv, p_l;
+  int4 *d_aproj = nullptr;  // per atom: its projectors {first, stride, count}
   int *d_pisa = nullptr, *d_pis = nullptr, *d_piv = nullptr, *d_pl = nullptr;
   double2 *d_P = nullptr, *d_Q = nullptr;
   double *d_H = nullptr, *d_nl = nullptr, *d_hn = nullptr, *d_D = nullptr, *d_dfnl = nullptr;
@@ -738,15 +741,21 @@ static int do_potential(amdk_ctx *c) {
 }
 
 static bool use_slice(const amdk_ctx *c);
-// The unpack of pairs [p0, p0+T) (kinetic term, occupation scaling) fused
-// with fnonloc for the first UNPACK_NPJ projectors; further projectors are
-// added in chunks (k_fnonloc_add).  pp/pm: +G/-G positions in the ray buffer.
-template <typename C> static void unpack_h(amdk_ctx *c, int p0, int T, const int *pp, const int *pm, long stride) {
+static int dg_nn(amdk_ctx *c, const void *A, int n1, const double *G, int n, double alpha, double beta, bool upper,
+                 void *out, bool g0twice = false);
+// The unpack of pairs [p0, p0+T) (kinetic term, occupation scaling) with
+// fnonloc: fused for up to UNPACK_NPJ projectors (their products then cost
+// less than another pass over C2), else C2 += P D as one FP64 tensor-core
+// product of all of them (256 projectors and 128 bands: 8 CUDA-core chunks
+// took 216 us per H|psi>, 70 us now; 128 and 512: 4.5 ms, 1.3 ms now).
+// pp/pm: +G/-G positions in the ray buffer.
+template <typename C> static int unpack_h(amdk_ctx *c, int p0, int T, const int *pp, const int *pm, long stride) {
   typedef decltype(C().x) Rl;
   const HostSetup &h = c->hs;
   const Geom &g = c->geom;
   const double scale = 1.0 / ((double)g.n1 * g.n2 * g.n3);
-  const int npj0 = std::min(c->nproj, UNPACK_NPJ);
+  const bool fused = c->nproj <= UNPACK_NPJ;
+  const int npj0 = fused ? c->nproj : 0;
   const int nb = std::min(2 * T, c->nstate - 2 * p0);
   // per-band maxima of C2 for its slicing (int8 products of the mixed path)
   unsigned long long *bmax = use_slice(c) ? c->d_c2max + 2 * p0 : nullptr;
@@ -755,18 +764,14 @@ template <typename C> static void unpack_h(amdk_ctx *c, int p0, int T, const int
   constexpr int PAIRS = unpack_pairs<C>();
   const dim3 gu(nblk(h.ngpw, 128), (T + PAIRS - 1) / PAIRS);
   k_unpack_fnonloc<C><<<gu, 128, (size_t)2 * PAIRS * npj0 * sizeof(Rl), c->st>>>(
-      h.ngpw, c->nstate, 2 * p0, T, npj0, pp, pm, (const C *)c->d_rb, stride, scale, c->d_hg, h.tpiba2,
-      c->d_occ, c->d_P, c->d_D, c->nproj, c->d_c0, c->d_c2, c->nproj > npj0 ? nullptr : bmax, 0);
-  // with projector chunks still to add, C2 is sliced from scratch
-  c->c2max_ok = bmax != nullptr && c->nproj <= npj0;
-  for (int j0 = npj0; j0 < c->nproj; j0 += UNPACK_NPJ) {
-    const int npj = std::min(UNPACK_NPJ, c->nproj - j0);
-    smem_opt_in<k_fnonloc_add<UNPACK_NPJ>>();
-    ++c->nlaunch;
-    const dim3 ga(nblk(h.ngpw, 128), (nb + FNL_BANDS - 1) / FNL_BANDS);
-    k_fnonloc_add<UNPACK_NPJ><<<ga, 128, (size_t)FNL_BANDS * npj * sizeof(double), c->st>>>(
-        h.ngpw, 2 * p0, nb, j0, npj, c->d_P, c->d_D, c->nproj, c->d_c2);
-  }
+      h.ngpw, c->nstate, 2 * p0, T, npj0, pp, pm, (const C *)c->d_rb, stride, scale, c->d_hg, h.tpiba2, c->d_occ, c->d_P,
+      c->d_D, c->nproj, c->d_c0, c->d_c2, fused ? bmax : nullptr, 0);
+  // with projectors still to add, C2 is sliced from scratch
+  c->c2max_ok = bmax != nullptr && fused;
+  if (!fused)
+    RC(dg_nn(c, c->d_P, c->nproj, c->d_D + (size_t)c->nproj * 2 * p0, nb, 1.0, 1.0, false,
+             c->d_c2 + (size_t)h.ngpw * 2 * p0, true));
+  return 0;
 }
 
 // vpsi + fnonloc: C2 = -f H C0 (C2 is written, not accumulated)
@@ -779,7 +784,7 @@ template <typename C> static int apply_h_t(amdk_ctx *c) {
       xt_bwd_pair<C>(c, p0, T);
       pencil_vpsi<C>(c, T, p0);
       xt_fwd<C>(c, T);
-      unpack_h<C>(c, p0, T, c->d_postp, c->d_postm, pencil_stride(c));
+      RC(unpack_h<C>(c, p0, T, c->d_postp, c->d_postm, pencil_stride(c)));
     }
     CK(cudaGetLastError());
     return 0;
@@ -798,7 +803,7 @@ template <typename C> static int apply_h_t(amdk_ctx *c) {
     z_pass<C, Z_VPSI>(c, 0, T, nullptr, nullptr);
     y_pass<C>(c, 0, -1, T);
     x_fwd<C>(c, 0, T);
-    unpack_h<C>(c, p0, T, c->d_posp, c->d_posm, rstride(c, 0));
+    RC(unpack_h<C>(c, p0, T, c->d_posp, c->d_posm, rstride(c, 0)));
   }
   CK(cudaGetLastError());
   return 0;
@@ -944,12 +949,13 @@ static void sg_nn(amdk_ctx *c, const double *B, double2 *out, int sub, bool digi
 
 // ------------------------------------------------- FP64 tensor-core GEMMs
 // 2D map of a column-major FP64 matrix, dim0 x dim1 (dim0 contiguous, the
-// leading dimension), box box0 x box1
-static int dg_encode(CUtensorMap *m, const void *base, long dim0, long dim1, int box0, int box1, CUtensorMapSwizzle sw) {
+// leading dimension unless ld is given), box box0 x box1
+static int dg_encode(CUtensorMap *m, const void *base, long dim0, long dim1, int box0, int box1, CUtensorMapSwizzle sw,
+                     long ld = 0) {
   PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
   if (!enc) return AMDK_ERR_CUDA;
   cuuint64_t dims[2] = {(cuuint64_t)dim0, (cuuint64_t)dim1};
-  cuuint64_t strides[1] = {(cuuint64_t)dim0 * sizeof(double)};
+  cuuint64_t strides[1] = {(cuuint64_t)(ld > 0 ? ld : dim0) * sizeof(double)};
   cuuint32_t box[2] = {(cuuint32_t)box0, (cuuint32_t)box1};
   cuuint32_t es[2] = {1, 1};
   if (enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<void *>(base), dims, strides, box, es,
@@ -960,10 +966,21 @@ static int dg_encode(CUtensorMap *m, const void *base, long dim0, long dim1, int
   }
   return 0;
 }
-// split-K partial tiles a TN product of m x n needs at most (buffer size)
+// blocks of a TN product of ntile output tiles and U (tile, k tile) units: all
+// resident, the same number on every SM, fewer only to keep 8 k tiles each (a
+// short block costs its pipeline fill and a partial tile to add).  Up to 3% of
+// the blocks are left out to make them a multiple of the tiles: the tiles' ranges
+// of k then coincide and share their operands in the L2 while they come in.
+static int dg_blocks(long U, int ntile, int nsm) {
+  const long all = (long)DG_TN_BPS * nsm, even = all / ntile * ntile;
+  return (int)std::max<long>(1, std::min(100 * even >= 97 * all ? even : all, U / 8));
+}
+// partial tiles per block: the output tiles its range can touch
+static int dg_seg(long U, int nb, int ktiles) { return (int)((U / nb + ktiles) / ktiles) + 1; }
+// partial tiles a TN product of m x n needs at most (buffer size)
 static size_t dg_part_doubles(const amdk_ctx *c, int m, int n) {
   const size_t ntile = (size_t)((m + DG_T - 1) / DG_T) * ((n + DG_T - 1) / DG_T);
-  return (2 * (size_t)c->nsm + ntile) * DG_T * DG_T;
+  return (ntile + 3 * (size_t)DG_TN_BPS * c->nsm) * DG_T * DG_T;
 }
 // out (m x n, leading dimension ldo) = alpha A^T B over the real index
 // K = 2 ngpw; A (K x m) and B (K x n) are the real views of complex band or
@@ -983,31 +1000,42 @@ static int dg_tn(amdk_ctx *c, const void *A, int m, const void *B, int n, double
   const int mt = (m + DG_T - 1) / DG_T, nt = (n + DG_T - 1) / DG_T;
   const int ntile = sym ? mt * (mt + 1) / 2 : mt * nt;
   const int ktiles = (int)((K + DG_KT - 1) / DG_KT);
-  // enough blocks to fill the GPU twice, but at least 8 k tiles each (a short
-  // block costs its pipeline fill, and every split is a partial tile to add)
-  int nsplit = std::max(1, std::min((ktiles + 7) / 8, (2 * c->nsm + ntile - 1) / ntile));
-  const int per = (ktiles + nsplit - 1) / nsplit;
-  nsplit = (ktiles + per - 1) / per;
+  const long U = (long)ntile * ktiles;
+  const int nb = dg_blocks(U, ntile, c->nsm), seg = dg_seg(U, nb, ktiles);
   c->nlaunch += 2;
-  k_dgemm_tn<<<dim3(ntile, nsplit), DG_THREADS, DG_TN_SMEM, st>>>(ta, tb, m, n, mt, sym ? 1 : 0, ktiles, per, c->d_dgpart,
-                                                                 c->d_info + 1, c->dg_plim);
+  k_dgemm_tn<<<nb, DG_THREADS, DG_TN_SMEM, st>>>(ta, tb, m, n, mt, sym ? 1 : 0, ntile, ktiles, seg, c->d_dgpart,
+                                                 c->d_info + 1, c->dg_plim);
   k_dgemm_tn_sum<<<(int)std::min<long>((long)ntile * (DG_T * DG_T / 32), 8L * c->nsm), 256, 0, st>>>(
-      c->d_dgpart, nsplit, ntile, mt, sym ? 1 : 0, m, n, alpha, out, ldo);
+      c->d_dgpart, nb, seg, ntile, ktiles, mt, sym ? 1 : 0, m, n, alpha, out, ldo);
   CK(cudaGetLastError());
   return 0;
 }
 // out (K x n, the real view of a complex band array) = alpha A G + beta out,
-// A the real view of n1 bands, G n1 x n (leading dimension n1); upper: G is
-// upper triangular (its lower part is not read)
+// A the real view of n1 bands (or projectors), G n1 x n (leading dimension
+// n1); upper: G is upper triangular (its lower part holds zeros); g0twice: A
+// holds half its value at G = 0
 static int dg_nn(amdk_ctx *c, const void *A, int n1, const double *G, int n, double alpha, double beta, bool upper,
-                 void *out) {
+                 void *out, bool g0twice) {
   const long K = 2L * c->hs.ngpw;
-  CUtensorMap ta;
-  RC(dg_encode(&ta, A, K, n1, 16, DG_NN_BS, CU_TENSOR_MAP_SWIZZLE_128B));
-  const long items = ((K + DG_NN_R - 1) / DG_NN_R) * ((n + DG_NN_J - 1) / DG_NN_J);
+  long ldg = n1;
+  if (n1 & 1) {
+    // TMA rows are a multiple of 16 bytes: an odd leading dimension is padded
+    ++ldg;
+    CK(cudaMemcpy2DAsync(c->d_gpad, sizeof(double) * ldg, G, sizeof(double) * n1, sizeof(double) * n1, n,
+                         cudaMemcpyDeviceToDevice, c->st));
+    G = c->d_gpad;
+  }
+  CUtensorMap ta, tg;
+  RC(dg_encode(&ta, A, K, n1, 16, DG_NN_K, CU_TENSOR_MAP_SWIZZLE_128B));
+  RC(dg_encode(&tg, G, n1, n, 8, DG_NN_J, CU_TENSOR_MAP_SWIZZLE_NONE, ldg));
+  // persistent blocks, two per SM; their number coprime to the column tiles, so
+  // that a block's items run through all of them (with upper they differ in work)
+  const long njt = (n + DG_NN_J - 1) / DG_NN_J, items = (K + DG_NN_R - 1) / DG_NN_R * njt;
+  long nb = 2L * c->nsm;
+  while (std::gcd(nb, njt) != 1) --nb;
   ++c->nlaunch;
-  k_dgemm_nn<<<(int)std::min<long>(items, c->nsm), DG_NN_THREADS, DG_NN_SMEM, c->st>>>(
-      ta, G, n1, K, n1, n, alpha, beta, upper ? 1 : 0, (double *)out, K, c->d_info + 1, c->dg_plim);
+  k_dgemm_nn<<<(int)std::min(items, nb), DG_NN_THREADS, DG_NN_SMEM, c->st>>>(
+      ta, tg, K, n1, n, alpha, beta, upper ? 1 : 0, g0twice ? 1 : 0, (double *)out, K, c->d_info + 1, c->dg_plim);
   CK(cudaGetLastError());
   return 0;
 }
@@ -1052,7 +1080,7 @@ static int energy_c0_terms(amdk_ctx *c) {
   RC(do_fnl(c));
   if (c->nproj) {
     ++c->nlaunch;
-    k_nl_energy_d<<<nblk((long)c->nproj * c->nstate), NTHR, 0, c->st>>>(c->nproj, c->nstate, c->d_H, c->d_nl, c->d_hn,
+    k_nl_energy_d<<<nblk((long)c->nproj * c->nstate), NTHR, 0, c->st>>>(c->nproj, c->nstate, c->d_pisa, c->d_aproj, c->d_H, c->d_nl, c->d_hn,
                                                                           c->d_occ, c->d_D, c->d_part,
                                                   c->d_scal + S_ENL, c->d_ticket + TK_ENL);
   } else {
@@ -1336,7 +1364,7 @@ static int do_ionic_forces(amdk_ctx *c) {
     }
   }
   ++c->nlaunch;
-  k_force_total<<<h.nat, NTHR, 0, c->st>>>(h.nat, c->nproj, c->nstate, c->d_pisa, c->d_hn, c->d_dfnl, c->d_occ, c->d_part,
+  k_force_total<<<h.nat, NTHR, 0, c->st>>>(h.nat, c->nproj, c->nstate, c->d_aproj, c->d_hn, c->d_dfnl, c->d_occ, c->d_part,
                                            pnb, c->d_isa_is, c->d_isa_ia, h.na_max, c->d_force);
   CK(cudaGetLastError());
   return 0;
@@ -1684,7 +1712,10 @@ static int build_device(amdk_ctx *c) {
   RC(c->alloc(&c->d_esr, 1));
   // projector list (isa-major within a species, as nl(isa,iv) of fnl)
   int isa0 = 0;
+  std::vector<int4> aproj;
   for (int is = 0; is < h.nsp; is++) {
+    for (int ia = 0; ia < h.na[is]; ia++)
+      aproj.push_back(make_int4((int)c->p_isa.size() + ia, h.na[is], h.ngh[is], 0));
     for (int iv = 0; iv < h.ngh[is]; iv++)
       for (int ia = 0; ia < h.na[is]; ia++) {
         c->p_isa.push_back(isa0 + ia);
@@ -1696,6 +1727,7 @@ static int build_device(amdk_ctx *c) {
   }
   c->nproj = (int)c->p_isa.size();
   if (c->nproj) {
+    RC(c->up(&c->d_aproj, aproj));
     RC(c->up(&c->d_pisa, c->p_isa));
     RC(c->up(&c->d_pis, c->p_is));
     RC(c->up(&c->d_piv, c->p_iv));
@@ -1730,6 +1762,7 @@ static int build_device(amdk_ctx *c) {
     const size_t np = dg_part_doubles(c, rows, h.nstate);
     RC(c->alloc(&c->d_dgpart, np));
     RC(c->alloc(&c->d_dgpart2, np));
+    if ((h.nstate | c->nproj) & 1) RC(c->alloc(&c->d_gpad, (size_t)(std::max(h.nstate, c->nproj) + 1) * h.nstate));
     CK(cudaFuncSetAttribute(k_dgemm_tn, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_TN_SMEM));
     CK(cudaFuncSetAttribute(k_dgemm_nn, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_NN_SMEM));
   }
@@ -1782,7 +1815,7 @@ template <typename C> static int seg_a_overlap(amdk_ctx *c) {
   CK(cudaMemcpyAsync(c->h_pin, c->d_scal, sizeof(double) * S_NSCAL, cudaMemcpyDeviceToHost, c->st));
   pencil_vpsi<C>(c, T);
   xt_fwd<C>(c, T);
-  unpack_h<C>(c, 0, T, c->d_postp, c->d_postm, pencil_stride(c));
+  RC(unpack_h<C>(c, 0, T, c->d_postp, c->d_postm, pencil_stride(c)));
   RC(do_gradient(c));
   CK(cudaMemcpyAsync(c->h_pin + S_NSCAL, c->d_scal + S_GMAX, sizeof(double), cudaMemcpyDeviceToHost, c->st));
   return 0;

@@ -11,32 +11,29 @@
 //
 // TN (out = alpha A^T B over the long real index K; A is K x m and B is
 // K x n, both column-major with leading dimension K): output tiles of 64 x 64,
-// the K range split over enough blocks to fill the GPU; one copy warp streams
-// 16-wide k tiles of A and B (128-byte swizzled TMA boxes of 16 x 64) through a
-// 4-stage mbarrier pipeline, four MMA warps each own a 32 x 32 quarter of the
-// tile.  The partial tiles go to a buffer that k_dgemm_tn_sum adds up in
-// split order (deterministic).  With sym only the tiles on and above the
-// diagonal are formed and the sum mirrors them (S is symmetric).
+// the (tile, 16-wide k tile) units split evenly over two blocks per SM; one
+// copy warp streams the k tiles of A and B (128-byte swizzled TMA boxes of
+// 16 x 64) through a 4-stage mbarrier pipeline, four MMA warps each own a
+// 32 x 32 quarter of the tile.  The partial tiles go to a buffer that
+// k_dgemm_tn_sum adds up in block order (deterministic).  With sym only the
+// tiles on and above the diagonal are formed and the sum mirrors them (S is
+// symmetric).
 //
 // NN (out = alpha A G + beta out; A is K x n1 column-major, G is n1 x n
 // column-major): persistent blocks over work items of 64 rows of the long
-// index x 128 output columns, eight warps each owning 32 rows x 32
-// columns; per 64-band half chunk, A arrives in four TMA boxes of 16 rows x
-// 64 bands through a 2-stage pipeline and the 64 x 128 slice of G by cp.async
-// into one of two buffers (kept for the whole kernel when G is at most
-// 128 x 128).  With upper, G is
-// upper triangular (U^{-1}): band blocks below a column block are skipped and
-// the lower part of G is read as zero.
+// index x 128 output columns, eight warps each owning 32 rows x 32 columns;
+// per 16-band step, A arrives in four TMA boxes and G in two, through a
+// 4-stage mbarrier pipeline.
 //
-// Fragment layouts (PTX ISA, mma.m8n8k4 with .f64): A (8 x 4, row) one value
-// per thread at row lane/4, column lane%4; B (4 x 8, col) row lane%4, column
-// lane/4; C (8 x 8) two values at row lane/4, columns 2 (lane%4) + {0, 1}.
+// Fragment layout (PTX ISA, mma.m16n8k8 with .f64): A (16 x 8) a0, a1 at rows
+// lane/4, lane/4 + 8 of column lane%4, a2, a3 the same of column lane%4 + 4; B
+// (8 x 8) rows lane%4, lane%4 + 4 of column lane/4; C (16 x 8) as two 8 x 8
+// blocks, rows lane/4 and lane/4 + 8, columns 2 (lane%4) + {0, 1}.
 // Each thread reads 16 bytes of shared memory at a time: in TN the two values
-// are consecutive k and serve two MMA steps (step s of half kb takes
-// k = 4 t + 2 kb + s, the same set for A and B, so that the eight lanes of a
-// quarter warp read eight different 16-byte bank groups of the swizzled
-// rows); in NN they are consecutive rows of the long index and serve two row
-// tiles (rows 2 g and 2 g + 1), from 128-byte-swizzled boxes as well.
+// are consecutive k and serve k = t and t + 4 of an MMA (half kb takes the k
+// tile's 4 t + 2 kb + {0, 1}, the same set for A and B, so that the eight lanes
+// of a quarter warp read eight different 16-byte bank groups of the swizzled
+// rows).
 //
 // Waits are bounded as in the integer-slice kernels: a pipeline wait gives up
 // after plim polls, sets *err and the shared abort flag; the block then runs
@@ -56,25 +53,18 @@ constexpr int DG_T = 64;    // TN output tile
 constexpr int DG_KT = 16;   // doubles per TN k tile (one 128-byte row)
 constexpr int DG_ST = 4;    // TN stages
 constexpr int DG_THREADS = 160;  // TN: 4 MMA warps + 1 copy warp
+constexpr int DG_TN_BPS = 2;     // TN blocks per SM (one: 110 us, two: 83, three: 83 for 128 x 128, K = 64 000)
 constexpr int DG_TN_STAGE = 2 * DG_T * DG_KT * 8;  // A and B boxes, 16 KB
 constexpr int DG_TN_SMEM = DG_ST * DG_TN_STAGE + 1024 + 2 * DG_ST * 8;
-constexpr int DG_NN_R = 64;    // rows of the long index per work item
-constexpr int DG_NN_B = 128;   // bands per staged G chunk
-constexpr int DG_NN_BS = 64;   // bands per A stage
+constexpr int DG_NN_R = 64;    // NN: rows of the long index per work item
 constexpr int DG_NN_J = 128;   // output columns per work item
-constexpr int DG_NN_GLD = DG_NN_BS + 8;  // padded row of a staged G slice (doubles): rows
-                                         // g and g + 1 half a bank line apart
-constexpr int DG_NN_ST = 2;
-constexpr int DG_NN_THREADS = 256;  // 8 MMA warps (thread 0 also issues the copies)
-constexpr int DG_NN_BOX = 16 * DG_NN_BS * 8;   // one TMA box, 16 rows x 64 bands, 8 KB
-constexpr int DG_NN_STAGE = 4 * DG_NN_BOX;     // 64 rows, 32 KB
-constexpr int DG_NN_SMEM = DG_NN_ST * DG_NN_STAGE + 2 * DG_NN_J * DG_NN_GLD * 8 + 1024 + 2 * DG_NN_ST * 8;
+constexpr int DG_NN_K = 16;    // bands per pipeline step
+constexpr int DG_NN_ST = 4;
+constexpr int DG_NN_THREADS = 256;             // 8 MMA warps (thread 0 also issues the TMA copies)
+constexpr int DG_NN_A = DG_NN_R * DG_NN_K * 8;  // 4 TMA boxes of 16 rows x 16 bands, 8 KB
+constexpr int DG_NN_STAGE = DG_NN_A + DG_NN_J * DG_NN_K * 8;
+constexpr int DG_NN_SMEM = DG_NN_ST * DG_NN_STAGE + 1024 + 2 * DG_NN_ST * 8;
 
-__device__ __forceinline__ void dg_mma(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
-}
 // 16 bytes (16-byte chunk `chunk` of row `row`) of a 128-byte-swizzled tile
 // of 128-byte rows (the tile 1024-byte aligned)
 __device__ __forceinline__ double2 dg_ld_sw(const unsigned char *tile, int row, int chunk) {
@@ -99,21 +89,41 @@ __host__ __device__ inline void dg_tile(int tile, int mt, int sym, int &it, int 
   }
 }
 
-// partial tiles: part[(split * ntile + tile) * 4096 + i + 64 j] =
-// sum over the split's k tiles of A[k][64 it + i] B[k][64 jt + j]
-__global__ void __launch_bounds__(DG_THREADS) k_dgemm_tn(const __grid_constant__ CUtensorMap ta,
-                                                         const __grid_constant__ CUtensorMap tb, int m, int n, int mt,
-                                                         int sym, int ktiles, int per, double *part, int *err,
-                                                         long plim) {
+__device__ __forceinline__ void dg_mma16(double (&d)[4], const double2 &a0, const double2 &a1, double b0, double b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+      : "d"(a0.x), "d"(a1.x), "d"(a0.y), "d"(a1.y), "d"(b0), "d"(b1));
+}
+
+// The (tile, k tile) units of a product, tile-major, are split into equal
+// contiguous ranges over nb blocks (all resident: every SM gets the same share
+// of the work); block b takes [b U / nb, (b+1) U / nb), U = ntile ktiles, and
+// leaves one partial tile per output tile it touches, in slots of its own:
+// part[(b seg + s) 4096 + i + 64 j], s the tile's place in its range.
+__host__ __device__ __forceinline__ int dg_first(int b, long U, int nb) { return (int)(b * U / nb); }
+// the block that holds unit u
+__host__ __device__ __forceinline__ int dg_block(long u, long U, int nb) {
+  const unsigned long x = (unsigned long)(u + 1) * nb - 1;
+  return (x >> 32) == 0 ? (int)((unsigned)x / (unsigned)U) : (int)(x / U);
+}
+// What bounds it: the FP64 tensor pipe (84% active where a block runs).  K =
+// 64 000, 128 x 128: 85 -> 83 us, symmetric 68 -> 66 us; K = 256 000,
+// 512 x 512: 6.6 -> 4.3 ms, symmetric 3.7 -> 2.4 ms (a grid of tiles x K
+// splits before, uneven over the SMs: 320 blocks of three resident per SM).
+__global__ void __launch_bounds__(DG_THREADS, 3) k_dgemm_tn(const __grid_constant__ CUtensorMap ta,
+                                                                    const __grid_constant__ CUtensorMap tb, int m, int n,
+                                                                    int mt, int sym, int ntile, int ktiles, int seg,
+                                                                    double *part, int *err, long plim) {
   extern __shared__ unsigned char dg_raw[];
   unsigned char *sm = dg_align1k(dg_raw);
   uint64_t *full = reinterpret_cast<uint64_t *>(sm + DG_ST * DG_TN_STAGE);
   uint64_t *empty = full + DG_ST;
   __shared__ int aborted;
   volatile int *ab = &aborted;
-  int it, jt;
-  dg_tile(blockIdx.x, mt, sym, it, jt);
-  const int k0 = blockIdx.y * per, nk = max(0, min(ktiles, k0 + per) - k0);
+  const long U = (long)ntile * ktiles;
+  const int u0 = dg_first(blockIdx.x, U, gridDim.x), u1 = dg_first(blockIdx.x + 1, U, gridDim.x), nk = u1 - u0;
+  const int tile0 = u0 / ktiles, kk0 = u0 - tile0 * ktiles;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     aborted = 0;
@@ -124,36 +134,50 @@ __global__ void __launch_bounds__(DG_THREADS) k_dgemm_tn(const __grid_constant__
     sg_bar_fence_init();
   }
   __syncthreads();
-  double acc[4][4][2];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
   if (warp == 4) {
     if (lane == 0) {
-      int issued = 0;
+      int issued = 0, tile = tile0, k = kk0, it, jt;
+      dg_tile(tile, mt, sym, it, jt);
       for (int q = 0; q < nk; ++q) {
         const int s = q % DG_ST;
         if (q >= DG_ST && !*ab && !sg_bar_wait(sg_smem(empty + s), ((q / DG_ST) - 1) & 1, err, 31, plim)) *ab = 1;
         if (*ab) break;
         unsigned char *st = sm + s * DG_TN_STAGE;
         sg_bar_expect_tx(sg_smem(full + s), DG_TN_STAGE);
-        sg_tma_2d(sg_smem(st), &ta, (k0 + q) * DG_KT, it * DG_T, sg_smem(full + s));
-        sg_tma_2d(sg_smem(st + DG_TN_STAGE / 2), &tb, (k0 + q) * DG_KT, jt * DG_T, sg_smem(full + s));
+        sg_tma_2d(sg_smem(st), &ta, k * DG_KT, it * DG_T, sg_smem(full + s));
+        sg_tma_2d(sg_smem(st + DG_TN_STAGE / 2), &tb, k * DG_KT, jt * DG_T, sg_smem(full + s));
         issued = q + 1;
+        if (++k == ktiles) {
+          k = 0;
+          if (++tile < ntile) dg_tile(tile, mt, sym, it, jt);
+        }
       }
       // no copy of this block may land after it exits
       for (int q = max(0, issued - DG_ST); q < issued; ++q)
         sg_bar_wait(sg_smem(full + q % DG_ST), (q / DG_ST) & 1, err, 32);
     }
-  } else {
-    const int wr = warp & 1, wc = warp >> 1, g = lane >> 2, t = lane & 3;
-    // a 32 x 32 quarter entirely outside m x n (few bands or projectors) has nothing to form
-    const bool live = it * DG_T + wr * 32 < m && jt * DG_T + wc * 32 < n;
-    for (int q = 0; q < nk; ++q) {
+    return;
+  }
+  const int wr = warp & 1, wc = warp >> 1, g = lane >> 2, t = lane & 3;
+  int q = 0;
+  for (int tile = tile0, k = kk0; q < nk; ++tile, k = 0) {
+    int it, jt;
+    dg_tile(tile, mt, sym, it, jt);
+    const int qe = min(nk, q + ktiles - k);
+    // a 16 x 8 piece entirely outside m x n (few bands or projectors) has nothing to form
+    const int ilive = min(2, (m - it * DG_T - wr * 32 + 15) / 16), jlive = min(4, (n - jt * DG_T - wc * 32 + 7) / 8);
+    double acc[2][4][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.0;
+    for (; q < qe; ++q) {
       const int s = q % DG_ST;
       if (!*ab && !sg_bar_wait(sg_smem(full + s), (q / DG_ST) & 1, err, 33, plim)) *ab = 1;
-      if (!*ab && live) {
+      __syncwarp();
+      if (!*ab && ilive > 0 && jlive > 0) {
         const unsigned char *A = sm + s * DG_TN_STAGE, *B = A + DG_TN_STAGE / 2;
 #pragma unroll
         for (int kb = 0; kb < 2; ++kb) {
@@ -162,71 +186,77 @@ __global__ void __launch_bounds__(DG_THREADS) k_dgemm_tn(const __grid_constant__
           for (int i = 0; i < 4; ++i) a[i] = dg_ld_sw(A, wr * 32 + i * 8 + g, 2 * t + kb);
 #pragma unroll
           for (int j = 0; j < 4; ++j) b[j] = dg_ld_sw(B, wc * 32 + j * 8 + g, 2 * t + kb);
-          // the two steps one after the other: 16 independent MMAs between
-          // the two that update one accumulator
+          if (ilive == 2 && jlive == 4) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
+            for (int j = 0; j < 4; ++j)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) dg_mma(acc[i][j], a[i].x, b[j].x);
+              for (int i = 0; i < 2; ++i) dg_mma16(acc[i][j], a[2 * i], a[2 * i + 1], b[j].x, b[j].y);
+          } else {
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
+            for (int j = 0; j < 4; ++j)
+              if (j < jlive)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) dg_mma(acc[i][j], a[i].y, b[j].y);
+                for (int i = 0; i < 2; ++i)
+                  if (i < ilive) dg_mma16(acc[i][j], a[2 * i], a[2 * i + 1], b[j].x, b[j].y);
+          }
         }
       }
       __syncwarp();
       if (lane == 0) sg_bar_arrive(sg_smem(empty + s));
     }
-  }
-  __syncthreads();
-  if (warp < 4) {
     const bool bad = *ab != 0;
-    const int wr = warp & 1, wc = warp >> 1, g = lane >> 2, t = lane & 3;
-    double *p = part + ((long)blockIdx.y * gridDim.x + blockIdx.x) * (DG_T * DG_T);
+    double *p = part + ((long)blockIdx.x * seg + (tile - tile0)) * (DG_T * DG_T);
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int r = wr * 32 + i * 8 + g, col = wc * 32 + j * 8 + 2 * t;
-        p[r + DG_T * col] = bad ? __longlong_as_double(0x7ff8000000000000LL) : acc[i][j][0];
-        p[r + DG_T * (col + 1)] = bad ? __longlong_as_double(0x7ff8000000000000LL) : acc[i][j][1];
-      }
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int r = wr * 32 + i * 16 + 8 * (e >> 1) + g, col = wc * 32 + j * 8 + 2 * t + (e & 1);
+          if (i < ilive && j < jlive) p[r + DG_T * col] = bad ? __longlong_as_double(0x7ff8000000000000LL) : acc[i][j][e];
+        }
   }
 }
 
-// out[i + ldo j] = alpha sum_split part (i < m, j < n).  A block takes 32
-// consecutive elements of the partial tiles; each of its 8 warps sums a
-// contiguous range of the splits in order, and warp 0 adds the 8 results in
-// order (deterministic).  With sym, an element of a tile above the diagonal
-// is written at (i, j) and (j, i).
-__global__ void __launch_bounds__(256) k_dgemm_tn_sum(const double *part, int nsplit, int ntile, int mt, int sym, int m,
-                                                      int n, double alpha, double *out, int ldo) {
+// out[i + ldo j] = alpha times the sum of the partial tiles of its tile (i < m,
+// j < n).  A block takes 32 consecutive elements of a tile; each of its 8 warps
+// sums a contiguous range of the blocks that hold the tile, in order (four
+// loads in flight), and warp 0 adds the 8 results in order (deterministic).
+// With sym, an element of a tile above the diagonal is written at (i, j) and
+// (j, i).
+__global__ void __launch_bounds__(256) k_dgemm_tn_sum(const double *part, int nb, int seg, int ntile, int ktiles, int mt,
+                                                      int sym, int m, int n, double alpha, double *out, int ldo) {
   __shared__ double red[8][32];
   const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
-  const long tot = (long)ntile * (DG_T * DG_T);
-  const int qn = (nsplit + 7) / 8, q0 = grp * qn, q1 = min(nsplit, q0 + qn);
+  const long tot = (long)ntile * (DG_T * DG_T), U = (long)ntile * ktiles;
   for (long base = (long)blockIdx.x * 32; base < tot; base += (long)gridDim.x * 32) {
-    const long e = base + lane;
-    double s0 = 0.0, s1 = 0.0;
-    int i = m, j = n, it = 0, jt = 0;
-    if (e < tot) {
-      const int tile = (int)(e / (DG_T * DG_T)), loc = (int)(e % (DG_T * DG_T));
-      dg_tile(tile, mt, sym, it, jt);
-      i = it * DG_T + loc % DG_T;
-      j = jt * DG_T + loc / DG_T;
-    }
-    if (i < m && j < n) {
-      const double *p = part + e;
+    const int tile = (int)(base / (DG_T * DG_T)), loc = (int)(base % (DG_T * DG_T)) + lane;
+    int it, jt;
+    dg_tile(tile, mt, sym, it, jt);
+    const int i = it * DG_T + loc % DG_T, j = jt * DG_T + loc / DG_T;
+    if (jt * DG_T + loc / DG_T >= n) continue;  // the same column for the whole block (32 divides 64)
+    const int b0 = dg_block((long)tile * ktiles, U, nb), b1 = dg_block((long)(tile + 1) * ktiles - 1, U, nb) + 1;
+    const int qn = (b1 - b0 + 7) / 8, q0 = b0 + grp * qn, q1 = min(b1, q0 + qn);
+    double s = 0.0;
+    if (i < m) {
+      // the tile is the first of every block's range but b0's, which may begin before it
+      const long bs = (long)seg * (DG_T * DG_T);
+      const double *p = part + loc;
       int q = q0;
-      for (; q + 1 < q1; q += 2) {
-        s0 += p[(long)q * tot];
-        s1 += p[(long)(q + 1) * tot];
+      if (grp == 0 && q < q1) s = p[(q++) * bs + (long)(tile - dg_first(b0, U, nb) / ktiles) * (DG_T * DG_T)];
+      auto at = [&](int b) { return p[b * bs]; };
+      for (; q + 3 < q1; q += 4) {
+        const double v0 = at(q), v1 = at(q + 1), v2 = at(q + 2), v3 = at(q + 3);
+        s += v0;
+        s += v1;
+        s += v2;
+        s += v3;
       }
-      if (q < q1) s0 += p[(long)q * tot];
+      for (; q < q1; ++q) s += at(q);
     }
-    red[grp][lane] = s0 + s1;
+    red[grp][lane] = s;
     __syncthreads();
-    if (grp == 0 && i < m && j < n) {
+    if (grp == 0 && i < m) {
       double v = red[0][lane];
 #pragma unroll
       for (int k = 1; k < 8; ++k) v += red[k][lane];
@@ -237,105 +267,60 @@ __global__ void __launch_bounds__(256) k_dgemm_tn_sum(const double *part, int ns
   }
 }
 
-// the MMAs of one band block for the column tiles C0 <= c < C1 of a warp; the
-// two steps one after the other, so that up to 16 independent MMAs separate
-// the two that update one accumulator
-template <int C0, int C1>
-__device__ __forceinline__ void dg_nn_cols(double (&acc)[2][2][4][2], const double2 (&a)[2][2], const double2 (&b)[4]) {
-#pragma unroll
-  for (int c = C0; c < C1; ++c)
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-      dg_mma(acc[p][0][c], a[p][0].x, b[c].x);
-      dg_mma(acc[p][1][c], a[p][0].y, b[c].x);
-    }
-#pragma unroll
-  for (int c = C0; c < C1; ++c)
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-      dg_mma(acc[p][0][c], a[p][1].x, b[c].y);
-      dg_mma(acc[p][1][c], a[p][1].y, b[c].y);
-    }
-}
-
-__device__ __forceinline__ void dg_cp8(uint32_t dst, const double *src, int bytes) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void dg_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void dg_cp_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-
 // out (K x n, leading dimension ldo) = alpha A G + beta out (beta 0: out is
-// only written).  ta maps A (K x n1, boxes of 16 rows x 64 bands); G is
-// n1 x n with leading dimension ldg; the boxes are 128-byte swizzled (the
-// 16-byte chunk of rows 2g, 2g + 1 of band b sits at chunk g ^ (b & 7)).
-// The work of a block is a sequence of units (work item, 64-band half chunk);
-// the A half chunk of a unit comes by TMA (thread 0 issues each load as soon
-// as every warp has released the stage it goes to), the matching 64 x 128
-// slice of G by cp.async into one of two buffers, the next unit's slice
-// copied while this unit multiplies.  When G has at most 128 rows and columns
-// both of its halves stay in the two buffers for the whole kernel.
-__global__ void __launch_bounds__(DG_NN_THREADS, 1) k_dgemm_nn(const __grid_constant__ CUtensorMap ta, const double *G,
-                                                               int ldg, long K, int n1, int n, double alpha,
-                                                               double beta, int upper, double *out, long ldo, int *err,
+// only written).  ta maps A (K x n1, boxes of 16 rows x 16 bands, 128-byte
+// swizzled), tg maps G (n1 x n, boxes of 8 bands x 128 columns).  With upper,
+// G is upper triangular (its lower part holds zeros) and the products with the
+// lower part are skipped 16 columns at a time.  With g0twice the product's
+// rows 0 and 1 (G = 0 of a projector matrix that holds half its value there)
+// count twice.
+// A warp's MMAs take the columns j as the M index and the long index r as N,
+// with the n index of two adjacent N tiles interleaved (r = 2n, 2n + 1), so
+// that a lane reads 16 bytes of every operand at a time, free of bank
+// conflicts (band k = t, t + 4 of an MMA step are 2t, 2t + 1 of a box's
+// eight), and owns four consecutive rows of an output column.
+// What bounds it: the FP64 tensor pipe.  Two blocks per SM, so that one's
+// epilogue (and its reads of the old outputs) runs under the other's MMAs; no
+// block-wide barrier in the loop: a warp waits for a stage's copies, and thread
+// 0 issues a stage's next copies once every warp has released it.  128 bands,
+// K = 64 000: C2 -= C0 Lambda 124 -> 108 us, C0 U^-1 86 -> 72 us; 512 bands,
+// K = 256 000: 8.6 -> 4.7 and 8.2 -> 2.5 ms (one block per SM, 64-band steps,
+// G copied in 8-byte pieces by all threads, a barrier per step, before).
+__global__ void __launch_bounds__(DG_NN_THREADS, 2) k_dgemm_nn(const __grid_constant__ CUtensorMap ta,
+                                                               const __grid_constant__ CUtensorMap tg, long K, int n1,
+                                                               int n, double alpha, double beta, int upper,
+                                                               int g0twice, double *out, long ldo, int *err,
                                                                long plim) {
   extern __shared__ unsigned char dg_raw[];
   unsigned char *sm = dg_align1k(dg_raw);
-  double *Gb = reinterpret_cast<double *>(sm + DG_NN_ST * DG_NN_STAGE);  // [2][128 columns][DG_NN_GLD]
-  uint64_t *full = reinterpret_cast<uint64_t *>(sm + DG_NN_ST * DG_NN_STAGE + 2 * DG_NN_J * DG_NN_GLD * 8);
-  uint64_t *empty = full + DG_NN_ST;
+  uint64_t *full = reinterpret_cast<uint64_t *>(sm + DG_NN_ST * DG_NN_STAGE), *empty = full + DG_NN_ST;
   __shared__ int aborted;
   volatile int *ab = &aborted;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nrt = (int)((K + DG_NN_R - 1) / DG_NN_R), njt = (n + DG_NN_J - 1) / DG_NN_J;
-  const int nbc = (n1 + DG_NN_B - 1) / DG_NN_B;
-  const long items = (long)nrt * njt;
-  const bool resident = njt == 1 && nbc == 1;
-  // G chunks of work item column tile jt (with upper only those at or above
-  // its column block), and the 64-band halves of chunk bc
-  auto chunks = [&](int jt) { return upper ? min(nbc, jt + 1) : nbc; };
-  auto halves = [&](int bc) { return min(2, (n1 - bc * DG_NN_B + DG_NN_BS - 1) / DG_NN_BS); };
-  // a cursor over the block's units
-  struct Cur {
-    long w;
-    int bc, hf;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int wj = warp >> 1, wr = warp & 1;  // 32 columns x 32 rows of the block's 128 x 64
+  const int nrt = (int)((K + DG_NN_R - 1) / DG_NN_R), njt = (n + DG_NN_J - 1) / DG_NN_J, items = nrt * njt;
+  auto steps = [&](int jt) {  // 16-band steps of a column tile
+    const int nb = upper ? min(n1, (jt + 1) * DG_NN_J) : n1;
+    return (nb + DG_NN_K - 1) / DG_NN_K;
   };
-  auto next = [&](Cur &u) {
-    if (++u.hf >= halves(u.bc)) {
-      u.hf = 0;
-      if (++u.bc >= chunks((int)(u.w % njt))) {
-        u.bc = 0;
-        u.w += gridDim.x;
-      }
-    }
-  };
-  // G slice of unit u into buffer buf (zero outside n1 x n and, with upper,
-  // below the diagonal); only whole 8-blocks that the products read
-  auto stage_g = [&](const Cur &u, int buf) {
-    const int jt = (int)(u.w % njt), b0 = u.bc * DG_NN_B + u.hf * DG_NN_BS;
-    const int jv = min(DG_NN_J, (n - jt * DG_NN_J + 7) / 8 * 8), bv = min(DG_NN_BS, (n1 - b0 + 7) / 8 * 8);
-    double *dst = Gb + (size_t)buf * DG_NN_J * DG_NN_GLD;
-    for (int e = threadIdx.x; e < jv * bv; e += DG_NN_THREADS) {
-      const int jl = e / bv, bl = e % bv;
-      const int b = b0 + bl, j = jt * DG_NN_J + jl;
-      const bool on = b < n1 && j < n && !(upper && b > j);
-      dg_cp8(sg_smem(dst + jl * DG_NN_GLD + bl), on ? G + b + (long)ldg * j : G, on ? 8 : 0);
-    }
-    dg_cp_commit();
-  };
-  // copy cursor (thread 0): the unit of the next A load
-  Cur cp{(long)blockIdx.x, 0, 0};
-  int issued = 0;
-  auto issue = [&]() {
-    const int s = issued % DG_NN_ST;
-    unsigned char *st = sm + s * DG_NN_STAGE;
-    const int rt = (int)(cp.w / njt);
-    sg_bar_expect_tx(sg_smem(full + s), DG_NN_STAGE);
+  // the block's work is a sequence of steps; thread 0's load cursor runs up to
+  // DG_NN_ST - 1 of them ahead
+  int lw = blockIdx.x, lk = 0, copies = 0;
+  auto load = [&]() {
+    const int lrt = lw / njt, ljt = lw - lrt * njt, st = copies % DG_NN_ST;
+    unsigned char *As = sm + st * DG_NN_STAGE, *Gs = As + DG_NN_A;
+    sg_bar_expect_tx(sg_smem(full + st), DG_NN_STAGE);
 #pragma unroll
-    for (int b4 = 0; b4 < 4; ++b4)
-      sg_tma_2d(sg_smem(st + b4 * DG_NN_BOX), &ta, rt * DG_NN_R + 16 * b4, cp.bc * DG_NN_B + cp.hf * DG_NN_BS,
-                sg_smem(full + s));
-    ++issued;
-    next(cp);
+    for (int i = 0; i < DG_NN_R / 16; ++i)
+      sg_tma_2d(sg_smem(As + i * 2048), &ta, lrt * DG_NN_R + 16 * i, lk * DG_NN_K, sg_smem(full + st));
+#pragma unroll
+    for (int i = 0; i < DG_NN_K / 8; ++i)
+      sg_tma_2d(sg_smem(Gs + i * DG_NN_J * 64), &tg, lk * DG_NN_K + 8 * i, ljt * DG_NN_J, sg_smem(full + st));
+    ++copies;
+    if (++lk >= steps(ljt)) {
+      lk = 0;
+      lw += gridDim.x;
+    }
   };
   if (threadIdx.x == 0) {
     aborted = 0;
@@ -344,138 +329,108 @@ __global__ void __launch_bounds__(DG_NN_THREADS, 1) k_dgemm_nn(const __grid_cons
       sg_bar_init(sg_smem(empty + s), DG_NN_THREADS / 32);
     }
     sg_bar_fence_init();
-    for (int k = 0; k < DG_NN_ST && cp.w < items; ++k) issue();
+    for (int s = 0; s < DG_NN_ST - 1 && lw < items; ++s) load();
   }
-  // G for the first unit (resident: both halves, for good)
-  Cur gu{(long)blockIdx.x, 0, 0};
-  if (gu.w < items) {
-    if (resident) {
-      for (int h = 0; h < halves(0); ++h) stage_g(Cur{gu.w, 0, h}, h);
-    } else {
-      stage_g(gu, 0);
-    }
-  }
-  const int wr = warp >> 2, wc = warp & 3, g = lane >> 2, t = lane & 3;
+  __syncthreads();
   int q = 0;
-  Cur gn = gu;  // the unit whose G slice is copied next (streaming)
-  if (!resident) next(gn);
-  for (long w = blockIdx.x; w < items; w += gridDim.x) {
-    const int rt = (int)(w / njt), jt = (int)(w % njt);
-    // column tiles of this warp with a column below n
-    const int clive = min(4, max(0, (n - jt * DG_NN_J - 8 * wc + 31) / 32));
-    double acc[2][2][4][2];
+  for (int w = blockIdx.x; w < items; w += gridDim.x) {
+    const int rt = w / njt, jt = w - rt * njt, j0 = jt * DG_NN_J + 32 * wj, nk = steps(jt);
+    // the item's old outputs towards the L2 while its products run
+    if (beta != 0.0)
+      for (int i = threadIdx.x; i < DG_NN_J * (DG_NN_R / 16); i += DG_NN_THREADS) {
+        const int j = jt * DG_NN_J + i / (DG_NN_R / 16);
+        const long r = (long)rt * DG_NN_R + 16 * (i % (DG_NN_R / 16));
+        if (j < n && r < K) asm volatile("prefetch.global.L2 [%0];" ::"l"(out + r + ldo * j));
+      }
+    double acc[2][2][2][4];  // [16 columns][16 rows][row parity][fragment]
 #pragma unroll
-    for (int p = 0; p < 2; ++p)
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int p = 0; p < 2; ++p)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[m][p][h][e] = 0.0;
+    for (int k = 0; k < nk; ++k, ++q) {
+      const int st = q % DG_NN_ST;
+      // the load DG_NN_ST - 1 steps ahead goes to the previous step's stage,
+      // once every warp has released it
+      if (threadIdx.x == 0 && lw < items && !*ab) {
+        if (q > 0 && !sg_bar_wait(sg_smem(empty + (q - 1) % DG_NN_ST), ((q - 1) / DG_NN_ST) & 1, err, 34, plim)) *ab = 1;
+        else load();
+      }
+      __syncwarp();
+      if (!*ab && !sg_bar_wait(sg_smem(full + st), (q / DG_NN_ST) & 1, err, 36, plim)) *ab = 1;
+      __syncwarp();
+      const unsigned char *As = sm + st * DG_NN_STAGE + wr * 4096;
+      const unsigned char *Gs = sm + st * DG_NN_STAGE + DG_NN_A + (32 * wj + g) * 64 + t * 16;
+      // live 16-column tiles: below n and, with upper, not left of these bands
+      const int jmin = upper ? k * DG_NN_K : 0;
+      const bool on0 = j0 < n && j0 + 15 >= jmin, on1 = j0 + 16 < n && j0 + 31 >= jmin;
+      if (!*ab && (on0 || on1)) {
+#pragma unroll
+        for (int kb = 0; kb < 2; ++kb) {
+          double2 a[2][2], b[2][2];
+#pragma unroll
+          for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+              a[m][h] = *reinterpret_cast<const double2 *>(Gs + (kb * DG_NN_J + 16 * m + 8 * h) * 64);
+#pragma unroll
+          for (int p = 0; p < 2; ++p)
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+              const int band = 8 * kb + 2 * t + s;
+              b[p][s] = *reinterpret_cast<const double2 *>(As + p * 2048 + band * 128 + ((g ^ (band & 7)) << 4));
+            }
+#pragma unroll
+          for (int m = 0; m < 2; ++m)
+            if (m == 0 ? on0 : on1)
+#pragma unroll
+              for (int p = 0; p < 2; ++p) {
+                dg_mma16(acc[m][p][0], a[m][0], a[m][1], b[p][0].x, b[p][1].x);
+                dg_mma16(acc[m][p][1], a[m][0], a[m][1], b[p][0].y, b[p][1].y);
+              }
+        }
+      }
+      __syncwarp();
+      if (lane == 0) sg_bar_arrive(sg_smem(empty + st));
+    }
+    // the eight old values of a 16-column tile are read before its stores
+    const bool bad = *ab != 0;
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const long r0 = (long)rt * DG_NN_R + 32 * wr + 4 * t;
+      double *o = out + r0 + ldo * (j0 + 16 * m + g);
+      double2 old[2][2][2];
 #pragma unroll
       for (int h = 0; h < 2; ++h)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[p][h][c][0] = acc[p][h][c][1] = 0.0;
-    // beta != 0: the output's old values, loaded now so that the item's
-    // products hide their latency
-    double2 old[2][4][2];
+        for (int p = 0; p < 2; ++p)
 #pragma unroll
-    for (int p = 0; p < 2; ++p)
+          for (int e = 0; e < 2; ++e)
+            old[h][p][e] = beta != 0.0 && j0 + 16 * m + 8 * h + g < n && r0 + 16 * p + 2 * e < K
+                               ? *reinterpret_cast<const double2 *>(o + ldo * (8 * h) + 16 * p + 2 * e)
+                               : make_double2(0.0, 0.0);
 #pragma unroll
-      for (int c = 0; c < 4; ++c)
+      for (int h = 0; h < 2; ++h)
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const long r = (long)rt * DG_NN_R + 32 * wr + 16 * p + 2 * g;
-          const int j = jt * DG_NN_J + 8 * (wc + 4 * c) + 2 * t + e;
-          old[p][c][e] = (beta != 0.0 && r < K && j < n) ? *reinterpret_cast<const double2 *>(out + r + ldo * j)
-                                                         : make_double2(0.0, 0.0);
-        }
-    for (int bc = 0; bc < chunks(jt); ++bc) {
-      for (int hf = 0; hf < halves(bc); ++hf, ++q) {
-        // this unit's G slice has landed (every thread's copies), and every
-        // warp is done with the previous unit, whose buffer the next copy reuses
-        dg_cp_wait_all();
-        __syncthreads();
-        if (!resident && gn.w < items) {
-          stage_g(gn, (q + 1) & 1);
-          next(gn);
-        }
-        const double *Gs = Gb + (size_t)(resident ? hf : (q & 1)) * DG_NN_J * DG_NN_GLD;
-        const int s = q % DG_NN_ST;
-        if (!*ab && !sg_bar_wait(sg_smem(full + s), (q / DG_NN_ST) & 1, err, 36, plim)) *ab = 1;
-        if (!*ab) {
-          const unsigned char *A = sm + s * DG_NN_STAGE + 2 * wr * DG_NN_BOX;
-          const int nkb = min(DG_NN_BS / 8, (n1 - bc * DG_NN_B - hf * DG_NN_BS + 7) / 8);
-#pragma unroll 2
-          for (int kb = 0; kb < nkb; ++kb) {
-            // band block of 8 (global index) against the column blocks of this warp
-            const int gkb = bc * (DG_NN_B / 8) + hf * (DG_NN_BS / 8) + kb;
-            double2 a[2][2], b[4];
+        for (int p = 0; p < 2; ++p)
 #pragma unroll
-            for (int p = 0; p < 2; ++p)
-#pragma unroll
-              for (int s2 = 0; s2 < 2; ++s2) {
-                const int band = 8 * kb + 2 * t + s2;
-                a[p][s2] = *reinterpret_cast<const double2 *>(A + p * DG_NN_BOX + band * 128 + ((g ^ (band & 7)) << 4));
-              }
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-              b[c] = *reinterpret_cast<const double2 *>(Gs + (8 * (wc + 4 * c) + g) * DG_NN_GLD + 8 * kb + 2 * t);
-            // with upper, column tile c takes this band block when its column
-            // block jt*16 + wc + 4c is not below it: the tiles c >= cmin;
-            // and the tiles c >= clive hold no column below n
-            int cmin = 0;
-            if (upper) cmin = min(4, max(0, (gkb - jt * (DG_NN_J / 8) - wc + 3) / 4));
-            switch (cmin * 5 + clive) {
-              case 1: dg_nn_cols<0, 1>(acc, a, b); break;
-              case 2: dg_nn_cols<0, 2>(acc, a, b); break;
-              case 3: dg_nn_cols<0, 3>(acc, a, b); break;
-              case 4: dg_nn_cols<0, 4>(acc, a, b); break;
-              case 7: dg_nn_cols<1, 2>(acc, a, b); break;
-              case 8: dg_nn_cols<1, 3>(acc, a, b); break;
-              case 9: dg_nn_cols<1, 4>(acc, a, b); break;
-              case 13: dg_nn_cols<2, 3>(acc, a, b); break;
-              case 14: dg_nn_cols<2, 4>(acc, a, b); break;
-              case 19: dg_nn_cols<3, 4>(acc, a, b); break;
-              default: break;  // no tile of this warp takes the block
-            }
+          for (int e = 0; e < 2; ++e) {
+            if (j0 + 16 * m + 8 * h + g >= n || r0 + 16 * p + 2 * e >= K) continue;
+            const double f = g0twice && r0 + 16 * p + e == 0 ? 2.0 * alpha : alpha;
+            double2 v = make_double2(f * acc[m][p][0][2 * h + e] + beta * old[h][p][e].x,
+                                     f * acc[m][p][1][2 * h + e] + beta * old[h][p][e].y);
+            if (bad) v.x = v.y = __longlong_as_double(0x7ff8000000000000LL);
+            *reinterpret_cast<double2 *>(o + ldo * (8 * h) + 16 * p + 2 * e) = v;
           }
-        }
-        __syncwarp();
-        if (lane == 0) sg_bar_arrive(sg_smem(empty + s));
-        if (threadIdx.x == 0 && cp.w < items && !*ab) {
-          // the next load goes to this stage once every warp has released
-          // it and this load has landed (no stage ever holds two copies)
-          if (!sg_bar_wait(sg_smem(empty + s), (q / DG_NN_ST) & 1, err, 34, plim) ||
-              !sg_bar_wait(sg_smem(full + s), (q / DG_NN_ST) & 1, err, 37))
-            *ab = 1;
-          else
-            issue();
-        }
-      }
-    }
-    // epilogue: rows r, r + 1 of column j as one 16-byte access
-    const bool bad = *ab != 0;
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-      const long r = (long)rt * DG_NN_R + 32 * wr + 16 * p + 2 * g;
-      if (r >= K) continue;
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int j = jt * DG_NN_J + 8 * (wc + 4 * c) + 2 * t + e;
-          if (j >= n) continue;
-          double2 v = make_double2(alpha * acc[p][0][c][e], alpha * acc[p][1][c][e]);
-          if (beta != 0.0) {
-            v.x += beta * old[p][c][e].x;
-            v.y += beta * old[p][c][e].y;
-          }
-          if (bad) v.x = v.y = __longlong_as_double(0x7ff8000000000000LL);
-          *reinterpret_cast<double2 *>(out + r + ldo * j) = v;
-        }
     }
   }
-  dg_cp_wait_all();
   // no copy of this block may land after it exits
-  if (threadIdx.x == 0)
-    for (int p = max(0, issued - DG_NN_ST); p < issued; ++p)
+  if (threadIdx.x == 0 && *ab)
+    for (int p = max(0, copies - DG_NN_ST); p < copies; ++p)
       sg_bar_wait(sg_smem(full + p % DG_NN_ST), (p / DG_NN_ST) & 1, err, 35);
-  __syncthreads();
 }
 
 }  // namespace amdk

@@ -624,45 +624,6 @@ __global__ void __launch_bounds__(128) k_unpack_fnonloc(int ngpw, int nstate, in
     }
   }
 }
-// fnonloc for projectors j0 .. j0+npj-1 beyond the first UNPACK_NPJ, FP64:
-// C2(b, G) += sum_j P_j(G) D(j, b) for bands band0 .. band0+nball-1; grid
-// (ngpw/128, ceil(nball/FNL_BANDS)), FNL_BANDS bands per block
-constexpr int FNL_BANDS = 16;
-template <int NPJ>
-__global__ void __launch_bounds__(128) k_fnonloc_add(int ngpw, int band0, int nball, int j0, int npj,
-                                                     const double2 *__restrict__ P, const double *__restrict__ D,
-                                                     int nproj, double2 *__restrict__ c2) {
-  extern __shared__ double Dsd[];  // [b][j]
-  band0 += blockIdx.y * FNL_BANDS;
-  const int nb = min(FNL_BANDS, nball - (int)blockIdx.y * FNL_BANDS);
-  for (int i = threadIdx.x; i < nb * npj; i += blockDim.x) {
-    const int b = i / npj, j = i - b * npj;
-    Dsd[i] = D[j0 + j + (long)nproj * (band0 + b)];
-  }
-  __syncthreads();
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= ngpw) return;
-  double2 pj[NPJ];
-#pragma unroll
-  for (int j = 0; j < NPJ; ++j) {
-    pj[j] = make_double2(0.0, 0.0);
-    if (j < npj) {
-      double2 v = P[(long)(j0 + j) * ngpw + g];
-      if (g == 0) v = make_double2(2.0 * v.x, 2.0 * v.y);
-      pj[j] = v;
-    }
-  }
-  for (int b = 0; b < nb; ++b) {
-    const double *d = Dsd + b * npj;
-    double2 a = make_double2(0.0, 0.0);
-#pragma unroll
-    for (int j = 0; j < NPJ; ++j)
-      if (j < npj) a = cfmas(pj[j], d[j], a);
-    double2 &o = c2[(long)(band0 + b) * ngpw + g];
-    o = make_double2(o.x + a.x, o.y + a.y);
-  }
-}
-
 // ---------------------------------------------------------------- bands
 // E_kin partial sums (total_energy.f90:38-61)
 // Band-major [nstate][ngpw] arrays in fixed contiguous chunks per block
@@ -1147,18 +1108,22 @@ __global__ void k_esr_par(int nat, const int *isa_is, const int *isa_ia, int na_
 
 // D = -f' (H nl), f' = occ (1 when < 1e-5)   (FNONLOC T = -FFI*WSG, UPF DDIA)
 // and E_nl partial: sum_b occ_b sum_j nl(j,b) (H nl)(j,b)
-// with (H nl)(j, b) = sum_j' H(j, j') nl(j', b) formed here (H couples the
-// projectors of one atom: wsg on the diagonal, or hlsg between projectors of
-// equal l and m) and stored for the forces
-__global__ void k_nl_energy_d(int nproj, int nstate, const double *H, const double *nl, double *hn, const double *occ,
-                              double *D, double *part, double *out, unsigned *ticket) {
+// with (H nl)(j, b) = sum_j' H(j, j') nl(j', b) formed here and stored for the
+// forces.  H couples the projectors of one atom only (wsg on the diagonal, or
+// hlsg between projectors of equal l and m): j' runs over those, first,
+// first + stride, ... of proj_of[atom] (256 projectors, 128 bands: 90 us with
+// the sum over all of them, 7 us now).
+__global__ void k_nl_energy_d(int nproj, int nstate, const int *proj_isa, const int4 *proj_of, const double *H,
+                              const double *nl, double *hn, const double *occ, double *D, double *part, double *out,
+                              unsigned *ticket) {
   double s = 0;
   long tot = (long)nproj * nstate;
   for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < tot; k += (long)gridDim.x * blockDim.x) {
     const int b = (int)(k / nproj), j = (int)(k - (long)b * nproj);
     const double *nb = nl + (long)nproj * b;
     double h = 0.0;
-    for (int jp = 0; jp < nproj; ++jp) h += H[j + (long)nproj * jp] * nb[jp];
+    const int4 po = proj_of[proj_isa[j]];
+    for (int i = 0, jp = po.x; i < po.z; ++i, jp += po.y) h += H[j + (long)nproj * jp] * nb[jp];
     hn[k] = h;
     double f = occ[b] < 1e-5 ? 1.0 : occ[b];
     D[k] = -f * h;
@@ -1267,16 +1232,18 @@ __global__ void k_dproj(int ngpw, int nproj, const double *gvec, const double2 *
 }
 // NLFOR / UPF_NLFOR (nuclear_grad.f90:51-89,153-199) plus POTFOR/e_sr sums:
 // F(isa) += potfor - sum_{j of isa} sum_b 2 occ_b (H nl)(j,b) dfnl_k(j,b)
-__global__ void k_force_total(int nat, int nproj, int nstate, const int *proj_isa, const double *hn, const double *dfnl,
+// proj_of[isa]: the atom's projectors, {first, stride, count} (64 atoms of 4
+// projectors: 255 us scanning all of them per atom, under 20 us now)
+__global__ void k_force_total(int nat, int nproj, int nstate, const int4 *proj_of, const double *hn, const double *dfnl,
                               const double *occ, const double *potpart, int pnb, const int *isa_is, const int *isa_ia,
                               int na_max, double *F) {
   __shared__ double sh[32];
   int a = blockIdx.x;
+  const int4 po = nproj ? proj_of[a] : make_int4(0, 0, 0, 0);
   for (int k = 0; k < 3; ++k) {
     double s = 0;
-    for (long q = threadIdx.x; q < (long)nproj * nstate; q += blockDim.x) {
-      int j = (int)(q % nproj), b = (int)(q / nproj);
-      if (proj_isa[j] != a) continue;
+    for (int q = threadIdx.x; q < po.z * nstate; q += blockDim.x) {
+      const int b = q / po.z, j = po.x + (q - b * po.z) * po.y;
       double w = occ[b];
       if (!(fabs(w) > 1e-12)) continue;
       s += 2.0 * w * hn[j + (long)nproj * b] * dfnl[(long)k * nproj + j + (long)3 * nproj * b];

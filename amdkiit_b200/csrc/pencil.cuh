@@ -351,7 +351,7 @@ constexpr int pencil_width(size_t csize, int n, int nc, int nt, int blocks, int 
   return 0;
 }
 constexpr int pencil_blocks(size_t csize, int nt) { return csize == 16 ? 512 / nt : (nt == 256 ? 3 : 2); }
-constexpr int pencil_tiles(int nc, int w) { return w > 0 ? (nc + w - 1) / w : 1 << 20; }
+constexpr int pencil_tiles(int nc, int w) { return w > 0 ? (nc + w - 1) / w : 4096; }
 // V(r)psi.  The whole plane (GA = 1) where a tile then still keeps half of a
 // block's threads busy, else one group of its columns at a time.
 template <typename C, int N> struct VpsiShape {
