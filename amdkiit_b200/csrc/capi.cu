@@ -126,7 +126,7 @@ struct amdk_ctx {
   void *d_vt2 = nullptr;
   double2 *d_c0 = nullptr, *d_c2 = nullptr, *d_cp = nullptr, *d_hnm1 = nullptr;
   double *d_rho = nullptr, *d_vpot = nullptr;
-  double2 *d_rhog = nullptr, *d_vg = nullptr, *d_vxg = nullptr, *d_fp = nullptr, *d_fm = nullptr, *d_cgrid = nullptr;
+  double2 *d_rhog = nullptr, *d_vg = nullptr, *d_vxg = nullptr, *d_fp = nullptr, *d_cgrid = nullptr;
   double *d_gam = nullptr, *d_uinv = nullptr;
   int *d_info = nullptr;
   double *d_part = nullptr, *d_scal = nullptr, *d_force = nullptr, *d_esr = nullptr, *d_fsr = nullptr;
@@ -259,6 +259,9 @@ static void prof_harvest(amdk_ctx *c) {
 
 
 static int nblk(long n, int t = NTHR) { return (int)std::min<long>((n + t - 1) / t, 1L << 30); }
+// blocks of a streaming kernel over n elements whose blocks end on a ticket: at
+// most `most`, and none without elements (4736 arrivals on one ticket take 6 us)
+static int sblk(long n, int most) { return (int)std::max<long>(1, std::min<long>(most, (n + NTHR - 1) / NTHR)); }
 
 template <typename C> static int make_plan(amdk_ctx *c, int n, Plan<C> &p) {
   int m = n, nf = 0;
@@ -318,7 +321,6 @@ template <typename C> static size_t yz_smem(int n) { return 2 * (size_t)n * TX *
 template <typename C> static void set_smem_attrs() {
   int mx = 227 * 1024;
   cudaFuncSetAttribute(k_x_bwd_pair<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_x_bwd_field<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
   cudaFuncSetAttribute(k_x_fwd<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
   cudaFuncSetAttribute(k_y<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
   cudaFuncSetAttribute(k_z<C, Z_TO_GRID>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
@@ -396,19 +398,19 @@ template <typename C> static void x_fwd(amdk_ctx *c, int sphere, int T, const XB
   prof_end(c);
 }
 
-// T fields on the density sphere (fp at +G, fm at -G) -> real or complex
+// T fields on the density sphere (SRC: see k_x_bwd_field) -> real or complex
 // grids (FP64 in and out; C is the precision of the transform itself)
-template <typename C = double2>
-static int field_to_grid(amdk_ctx *c, int T, const double2 *fp, const double2 *fm, double2 *cgrid,
+template <typename C = double2, int SRC = FS_REAL>
+static int field_to_grid(amdk_ctx *c, int T, const double2 *f, double2 *cgrid,
                          const XBufs &b = XBufs{}) {
   const Geom &g = c->geom;
   long lines = (long)T * g.nray[1];
   ++c->nlaunch;
   with_n(g.n1, [&](auto NC) {
     constexpr int N = decltype(NC)::value;
-    smem_opt_in<k_x_bwd_field<C, N>>();
-    k_x_bwd_field<C, N><<<nblk(lines, LX), NTHR, x_smem<C>(g.n1), c->st>>>(fp, fm, g.ngrho, 1, T, g, plan<C>(c, 0),
-                                                                         (C *)rays_of(c, 1, b));
+    smem_opt_in<k_x_bwd_field<C, N, SRC>>();
+    k_x_bwd_field<C, N, SRC><<<nblk(lines, LX), NTHR, x_smem<C>(g.n1), c->st>>>(
+        f, c->d_gvec, c->hs.tpiba, g.ngrho, 1, T, g, plan<C>(c, 0), (C *)rays_of(c, 1, b));
   });
   y_pass<C>(c, 1, +1, T, b);
   z_pass<C, Z_TO_GRID>(c, 1, T, cgrid, nullptr, 0, b);
@@ -623,7 +625,7 @@ template <typename C> static int density_pairs_t(amdk_ctx *c) {
 template <typename C> static int rhor2g_t(amdk_ctx *c) {
   const HostSetup &h = c->hs;
   const Geom &g = c->geom;
-  RC(grid_to_rays<C>(c, 1, nullptr, c->d_rho));
+  RC(grid_to_rays<C>(c, 1, nullptr, c->d_rho));  // left there by the iteration, whose k_vloc_g gathers rho(G)
   double scale = 1.0 / ((double)g.n1 * g.n2 * g.n3);
   ++c->nlaunch;
   k_gather_p<C><<<nblk(h.ngrho), NTHR, 0, c->st>>>(h.ngrho, c->d_posp, (C *)c->d_rbf, scale, c->d_rhog);
@@ -645,16 +647,17 @@ static int do_density(amdk_ctx *c) {
 static int store_potential(amdk_ctx *c, const double2 *grid, double *vpot, void *vt) {
   const Geom &g = c->geom;
   const long npt = (long)g.n1 * g.n2 * g.n3;
-  CK(cudaMemcpy2DAsync(vpot, sizeof(double), grid, sizeof(double2), sizeof(double), npt, cudaMemcpyDeviceToDevice,
-                       c->st));
-  if (c->pencil_vpsi) {
+  if (!c->pencil_vpsi) {
+    CK(cudaMemcpy2DAsync(vpot, sizeof(double), grid, sizeof(double2), sizeof(double), npt, cudaMemcpyDeviceToDevice,
+                         c->st));
+  } else {
     dim3 gt((g.n1 + 31) / 32, (g.n1 + 31) / 32, g.n1);
     const int n1f = fft_n1(g.n1), n2f = g.n1 / n1f;
     ++c->nlaunch;
     if (c->precision == AMDK_MIXED)
-      k_v_permute<float><<<gt, dim3(32, 8), 0, c->st>>>(g.n1, g.n1, n1f, n2f, vpot, (float *)vt);
+      k_v_store<float><<<gt, dim3(32, 8), 0, c->st>>>(g.n1, n1f, n2f, grid, vpot, (float *)vt);
     else
-      k_v_permute<double><<<gt, dim3(32, 8), 0, c->st>>>(g.n1, g.n1, n1f, n2f, vpot, (double *)vt);
+      k_v_store<double><<<gt, dim3(32, 8), 0, c->st>>>(g.n1, n1f, n2f, grid, vpot, (double *)vt);
   }
   return 0;
 }
@@ -670,25 +673,23 @@ template <typename C> static int potential_lsd_t(amdk_ctx *c) {
   double2 *g0 = c->d_cgrid, *g1 = c->d_cgrid + npt;
   ++c->nlaunch;
   if (sizeof(C) == sizeof(float2))
-    k_xc_lsd<float><<<RED_BLOCKS, NTHR, 0, c->st>>>(npt, c->d_rho, c->d_rho2, g0, g1, c->d_part, c->d_scal + S_EXC,
+    k_xc_lsd<float><<<sblk(npt, RED_BLOCKS), NTHR, 0, c->st>>>(npt, c->d_rho, c->d_rho2, g0, g1, c->d_part, c->d_scal + S_EXC,
                                                    c->d_ticket + TK_XC);
   else
-    k_xc_lsd<double><<<RED_BLOCKS, NTHR, 0, c->st>>>(npt, c->d_rho, c->d_rho2, g0, g1, c->d_part,
+    k_xc_lsd<double><<<sblk(npt, RED_BLOCKS), NTHR, 0, c->st>>>(npt, c->d_rho, c->d_rho2, g0, g1, c->d_part,
                                                     c->d_scal + S_EXC, c->d_ticket + TK_XC);
   RC(grid_to_rays<C>(c, 2, c->d_cgrid, nullptr));
   const double scale = 1.0 / (double)npt;
   // both spins' G-space potentials first (the ray buffer holds both fields)
-  double2 *vx[2] = {c->d_vxg, c->d_fp + h.ngrho}, *vm[2] = {c->d_fm, c->d_fm + h.ngrho};
+  double2 *vx[2] = {c->d_vxg, c->d_fp + h.ngrho};
   for (int sp = 0; sp < 2; ++sp) {
     ++c->nlaunch;
     k_xc_combine<C><<<nblk(h.ngrho), NTHR, 0, c->st>>>(h.ngrho, 0, c->d_posp, c->d_posm,
                                                        (const C *)c->d_rbf + (size_t)sp * rstride(c, 1), rstride(c, 1),
                                                        scale, c->d_gvec, h.tpiba, c->d_vg, vx[sp]);
-    ++c->nlaunch;
-    k_conj_field<<<nblk(h.ngrho), NTHR, 0, c->st>>>(h.ngrho, vx[sp], vm[sp]);
   }
   for (int sp = 0; sp < 2; ++sp) {
-    RC(field_to_grid<C>(c, 1, vx[sp], vm[sp], c->d_cgrid));
+    RC(field_to_grid<C>(c, 1, vx[sp], c->d_cgrid));
     RC(store_potential(c, c->d_cgrid, sp ? c->d_vpot2 : c->d_vpot, sp ? c->d_vt2 : c->d_vt));
   }
   CK(cudaGetLastError());
@@ -697,38 +698,41 @@ template <typename C> static int potential_lsd_t(amdk_ctx *c) {
 
 // eval_pot + cal_vpot_ex; the density-sphere transforms run in the pair
 // transforms' precision (FP32 on the mixed path, which ends on FP64)
-template <typename C> static int potential_t(amdk_ctx *c) {
+// (gather: rho's forward transform is in the ray buffer, rho(G) is taken from
+// there and stored)
+template <typename C> static int potential_t(amdk_ctx *c, bool gather = false) {
   const HostSetup &h = c->hs;
   const Geom &g = c->geom;
   long npt = (long)g.n1 * g.n2 * g.n3;
   // eval_pot in G space and E_H, E_loc sums
   ++c->nlaunch;
-  k_vloc_g<<<RED_BLOCKS, NTHR, 0, c->st>>>(h.ngrho, c->d_hg, h.tpiba2, c->d_rhog, c->d_erhos, c->d_evps, c->d_vg,
-                                           c->d_part, c->d_scal + S_EH, c->d_ticket + TK_VLOC);
+  auto vloc = [&](auto K) {
+    K<<<sblk(h.ngrho, RED_BLOCKS), NTHR, 0, c->st>>>(h.ngrho, c->d_posp, (const C *)c->d_rbf, 1.0 / (double)npt, c->d_hg, h.tpiba2,
+                                      c->d_rhog, c->d_erhos, c->d_evps, c->d_vg, c->d_part, c->d_scal + S_EH,
+                                      c->d_ticket + TK_VLOC);
+  };
+  if (gather) vloc(k_vloc_g<C, true>);
+  else vloc(k_vloc_g<C, false>);
   int gga = (h.xc == AMDK_XC_PBE);
   double2 *g0 = c->d_cgrid, *g1 = c->d_cgrid + npt;
   if (h.lsd) return potential_lsd_t<C>(c);
   if (gga) {
-    ++c->nlaunch;
-    k_grad_fields<<<nblk(h.ngrho), NTHR, 0, c->st>>>(h.ngrho, c->d_gvec, h.tpiba, c->d_rhog, c->d_fp, c->d_fm);
-    RC(field_to_grid<C>(c, 2, c->d_fp, c->d_fm, c->d_cgrid));
+    RC((field_to_grid<C, FS_GRAD>(c, 2, c->d_rhog, c->d_cgrid)));
   }
   ++c->nlaunch;
   // the functional in the transforms' precision (FP32 on the mixed path)
   if (sizeof(C) == sizeof(float2))
-    k_xc<float><<<RED_BLOCKS, NTHR, 0, c->st>>>(npt, h.xc, c->d_rho, g0, g1, c->d_part, c->d_scal + S_EXC,
+    k_xc<float><<<sblk(npt, RED_BLOCKS), NTHR, 0, c->st>>>(npt, h.xc, c->d_rho, g0, g1, c->d_part, c->d_scal + S_EXC,
                                                c->d_ticket + TK_XC);
   else
-    k_xc<double><<<RED_BLOCKS, NTHR, 0, c->st>>>(npt, h.xc, c->d_rho, g0, g1, c->d_part, c->d_scal + S_EXC,
+    k_xc<double><<<sblk(npt, RED_BLOCKS), NTHR, 0, c->st>>>(npt, h.xc, c->d_rho, g0, g1, c->d_part, c->d_scal + S_EXC,
                                                 c->d_ticket + TK_XC);
   RC(grid_to_rays<C>(c, gga ? 2 : 1, c->d_cgrid, nullptr));
   double scale = 1.0 / (double)npt;
   ++c->nlaunch;
   k_xc_combine<C><<<nblk(h.ngrho), NTHR, 0, c->st>>>(h.ngrho, gga, c->d_posp, c->d_posm, (C *)c->d_rbf, rstride(c, 1),
                                                      scale, c->d_gvec, h.tpiba, c->d_vg, c->d_vxg);
-  ++c->nlaunch;
-  k_conj_field<<<nblk(h.ngrho), NTHR, 0, c->st>>>(h.ngrho, c->d_vxg, c->d_fm);
-  RC(field_to_grid<C>(c, 1, c->d_vxg, c->d_fm, c->d_cgrid));
+  RC(field_to_grid<C>(c, 1, c->d_vxg, c->d_cgrid));
   // V(r) = Re of the backward transform (xc.f90:299-301), and V in the
   // x-plane-major layout the pencil kernel reads
   RC(store_potential(c, c->d_cgrid, c->d_vpot, c->d_vt));
@@ -742,7 +746,7 @@ static int do_potential(amdk_ctx *c) {
 
 static bool use_slice(const amdk_ctx *c);
 static int dg_nn(amdk_ctx *c, const void *A, int n1, const double *G, int n, double alpha, double beta, bool upper,
-                 void *out, bool g0twice = false);
+                 void *out, bool g0twice = false, bool zclean = false);
 // The unpack of pairs [p0, p0+T) (kinetic term, occupation scaling) with
 // fnonloc: fused for up to UNPACK_NPJ projectors (their products then cost
 // less than another pass over C2), else C2 += P D as one FP64 tensor-core
@@ -894,7 +898,7 @@ static void sg_slice(amdk_ctx *c, const double2 *x, int8_t *planes, double *scal
 // out (nm x n, leading dimension ldo) = alpha diag(sa) A B^T diag(sb), the
 // product over the real index; n = nstate columns (B = C0 or C2 planes)
 static void sg_tn(amdk_ctx *c, const CUtensorMap &ta, const CUtensorMap &tb, int same, const double *sa,
-                  const double *sb, double alpha, double *out, int nm = -1, int ldo = -1) {
+                  const double *sb, double alpha, double *out, int nm = -1, int ldo = -1, const G0Term &g0 = G0Term{}) {
   const int n = c->nstate;
   if (nm < 0) nm = n;
   if (ldo < 0) ldo = n;
@@ -902,7 +906,7 @@ static void sg_tn(amdk_ctx *c, const CUtensorMap &ta, const CUtensorMap &tb, int
   k_sgemm_tn<SG_S><<<c->sg_chunks, SG_TN_THREADS, SgTn<SG_S>::SMEM, c->st>>>(ta, tb, same, c->sg_ktiles, c->sg_per, c->d_sgpart,
                                                                      c->d_sgerr, c->sg_plim);
   k_sgemm_reduce<<<n, SG_RG * SG_M, 0, c->st>>>(c->sg_chunks, c->d_sgpart, nm, sa, sb, same ? c->d_sgnsq : nullptr,
-                                            alpha, out, ldo);
+                                            alpha, out, ldo, g0);
 }
 // projector planes: set up once the projector count is known (mixed-capable
 // contexts with slice products)
@@ -987,7 +991,7 @@ static size_t dg_part_doubles(const amdk_ctx *c, int m, int n) {
 // projector arrays.  sym: B = A, only the upper tiles are formed and the
 // result is mirrored.
 static int dg_tn(amdk_ctx *c, const void *A, int m, const void *B, int n, double alpha, double *out, int ldo,
-                 bool sym = false, long Kin = 0, cudaStream_t sin = nullptr) {
+                 bool sym = false, const G0Term &g0 = G0Term{}, long Kin = 0, cudaStream_t sin = nullptr) {
   // K: 2 ngpw unless given (a slab rank's 2 ngpw_local); stream: the context's unless given
   const long K = Kin > 0 ? Kin : 2L * c->hs.ngpw;
   cudaStream_t st = sin ? sin : c->st;
@@ -1006,16 +1010,16 @@ static int dg_tn(amdk_ctx *c, const void *A, int m, const void *B, int n, double
   k_dgemm_tn<<<nb, DG_THREADS, DG_TN_SMEM, st>>>(ta, tb, m, n, mt, sym ? 1 : 0, ntile, ktiles, seg, c->d_dgpart,
                                                  c->d_info + 1, c->dg_plim);
   k_dgemm_tn_sum<<<(int)std::min<long>((long)ntile * (DG_T * DG_T / 32), 8L * c->nsm), 256, 0, st>>>(
-      c->d_dgpart, nb, seg, ntile, ktiles, mt, sym ? 1 : 0, m, n, alpha, out, ldo);
+      c->d_dgpart, nb, seg, ntile, ktiles, mt, sym ? 1 : 0, m, n, alpha, out, ldo, g0);
   CK(cudaGetLastError());
   return 0;
 }
 // out (K x n, the real view of a complex band array) = alpha A G + beta out,
 // A the real view of n1 bands (or projectors), G n1 x n (leading dimension
 // n1); upper: G is upper triangular (its lower part holds zeros); g0twice: A
-// holds half its value at G = 0
+// holds half its value at G = 0; zclean: Im out(G = 0) = 0
 static int dg_nn(amdk_ctx *c, const void *A, int n1, const double *G, int n, double alpha, double beta, bool upper,
-                 void *out, bool g0twice) {
+                 void *out, bool g0twice, bool zclean) {
   const long K = 2L * c->hs.ngpw;
   long ldg = n1;
   if (n1 & 1) {
@@ -1035,7 +1039,7 @@ static int dg_nn(amdk_ctx *c, const void *A, int n1, const double *G, int n, dou
   while (std::gcd(nb, njt) != 1) --nb;
   ++c->nlaunch;
   k_dgemm_nn<<<(int)std::min(items, nb), DG_NN_THREADS, DG_NN_SMEM, c->st>>>(
-      ta, tg, K, n1, n, alpha, beta, upper ? 1 : 0, g0twice ? 1 : 0, (double *)out, K, c->d_info + 1, c->dg_plim);
+      ta, tg, K, n1, n, alpha, beta, upper ? 1 : 0, g0twice ? 1 : 0, zclean ? 1 : 0, (double *)out, K, c->d_info + 1, c->dg_plim);
   CK(cudaGetLastError());
   return 0;
 }
@@ -1087,7 +1091,7 @@ static int energy_c0_terms(amdk_ctx *c) {
     CK(cudaMemsetAsync(c->d_scal + S_ENL, 0, sizeof(double), c->st));
   }
   ++c->nlaunch;
-  k_ekin<<<c->red_ekin, NTHR, 0, c->st>>>(h.ngpw, c->nstate, c->d_c0, c->d_hg, c->d_occ, c->d_part,
+  k_ekin<<<sblk((long)h.ngpw * c->nstate, c->red_ekin), NTHR, 0, c->st>>>(h.ngpw, c->nstate, c->d_c0, c->d_hg, c->d_occ, c->d_part,
                                          c->d_scal + S_EKIN, c->d_ticket + TK_EKIN);
   return 0;
 }
@@ -1118,7 +1122,7 @@ static int n_occupied(const amdk_ctx *c) {
 // one pass: S_GMAX and S_GG
 static void gmax_precon(amdk_ctx *c) {
   ++c->nlaunch;
-  k_gmax_precon<<<c->red_gmax, NTHR, 0, c->st>>>(c->hs.ngpw, n_occupied(c), c->d_vpp, c->d_occ, c->d_c2, c->d_part,
+  k_gmax_precon<<<sblk((long)c->hs.ngpw * n_occupied(c), c->red_gmax), NTHR, 0, c->st>>>(c->hs.ngpw, n_occupied(c), c->d_vpp, c->d_occ, c->d_c2, c->d_part,
                                                 c->d_scal + S_GMAX, c->d_ticket + TK_GRAD);
 }
 
@@ -1131,10 +1135,19 @@ static void spin_mask(amdk_ctx *c, double *A) {
   k_spin_mask<<<nblk((long)n * n), NTHR, 0, c->st>>>(n, c->hs.nel_up, A);
 }
 
+// the G = 0 term of 2 Re a^H b between band arrays
+static G0Term g0_term(const amdk_ctx *c, const double2 *a, const double2 *b, const double *occ = nullptr) {
+  G0Term g;
+  g.a = (const double *)a;
+  g.b = (const double *)b;
+  g.occ = occ;
+  g.ld = 2L * c->hs.ngpw;
+  return g;
+}
 static int do_gradient(amdk_ctx *c) {
-  const HostSetup &h = c->hs;
   const int n = c->nstate;
   const bool sl = use_slice(c);
+  const G0Term g0 = g0_term(c, c->d_c2, c->d_c0, c->d_occ);
   if (sl) {
     if (c->c2max_ok) {
       // the unpack recorded C2's band maxima: only the digit pass
@@ -1147,40 +1160,35 @@ static int do_gradient(amdk_ctx *c) {
     }
     // C0's planes are those the last orthonormalisation wrote, if C0 has not changed since
     if (c->sg_c0_buf != (void *)c->d_c0) sg_slice(c, c->d_c0, c->d_plA, c->d_sgA);
-    sg_tn(c, c->tm_b_tn, c->tm_a_tn, 0, c->d_sgB, c->d_sgA, 2.0, c->d_gam);
+    sg_tn(c, c->tm_b_tn, c->tm_a_tn, 0, c->d_sgB, c->d_sgA, 2.0, c->d_gam, n, n, g0);
   } else {
-    RC(dg_tn(c, c->d_c2, n, c->d_c0, n, 2.0, c->d_gam, n));
+    RC(dg_tn(c, c->d_c2, n, c->d_c0, n, 2.0, c->d_gam, n, false, g0));
   }
-  ++c->nlaunch;
-  k_g0_correct<<<dim3(nblk(n), n), NTHR, 0, c->st>>>(n, h.ngpw, c->d_c2, c->d_c0, c->d_gam, c->d_occ, 1, 0);
   spin_mask(c, c->d_gam);
   if (sl)
     sg_nn(c, c->d_gam, c->d_c2, 1, false);
   else
-    RC(dg_nn(c, c->d_c0, n, c->d_gam, n, -1.0, 1.0, false, c->d_c2));
-  ++c->nlaunch;
-  k_zclean<<<nblk(n), NTHR, 0, c->st>>>(n, h.ngpw, c->d_c2);
+    RC(dg_nn(c, c->d_c0, n, c->d_gam, n, -1.0, 1.0, false, c->d_c2, false, true));
   c->c2max_ok = false;  // C2 is the projected gradient now
   gmax_precon(c);
   CK(cudaGetLastError());
   return 0;
 }
 
-// PCG; the step number goes through pinned host memory and the S_ISTEP slot
-// so that a captured graph of this step reads the current one.  The
-// gradient norm S_GG is the one do_gradient left for the current C2
-// (recompute: form it here, for a caller that changed C2 since).
-static int do_pcg(amdk_ctx *c, int istep, bool recompute = false) {
+// the CG step number, from pinned host memory (h_pin[S_NSCAL + 1], set before
+// the launch, so that a captured graph of this copy takes the current one)
+static int copy_istep(amdk_ctx *c) {
+  CK(cudaMemcpyAsync(c->d_scal + S_ISTEP, c->h_pin + S_NSCAL + 1, sizeof(double), cudaMemcpyHostToDevice, c->st));
+  return 0;
+}
+// PCG with the step number in S_ISTEP and the gradient norm S_GG of the
+// current C2 (left by do_gradient, or formed by the caller)
+static int do_pcg(amdk_ctx *c) {
   const HostSetup &h = c->hs;
   c->sg_c0_buf = nullptr;  // C0 changes in place
-  c->h_pin[S_NSCAL + 1] = (double)istep;
-  CK(cudaMemcpyAsync(c->d_scal + S_ISTEP, c->h_pin + S_NSCAL + 1, sizeof(double), cudaMemcpyHostToDevice, c->st));
-  if (recompute) gmax_precon(c);
   ++c->nlaunch;
-  k_pcg_update<<<RED_BLOCKS * 4, NTHR, 0, c->st>>>(h.ngpw, c->nstate, c->d_scal, c->d_vpp, c->d_occ, c->d_c2, c->d_hnm1,
-                                                   c->d_c0);
-  ++c->nlaunch;
-  k_copy_scalar<<<1, 1, 0, c->st>>>(c->d_scal + S_GG, c->d_scal + S_GGPREV);
+  k_pcg_update<<<sblk((long)h.ngpw * c->nstate, RED_BLOCKS * 4), NTHR, 0, c->st>>>(h.ngpw, c->nstate, c->d_scal, c->d_ticket + TK_PCG, c->d_vpp, c->d_occ,
+                                                   c->d_c2, c->d_hnm1, c->d_c0);
   CK(cudaGetLastError());
   return 0;
 }
@@ -1255,18 +1263,16 @@ static int chol_inv_blocked(amdk_ctx *c, int n) {
 }
 
 static int do_ortho(amdk_ctx *c, bool check = true, bool swap = true) {
-  const HostSetup &h = c->hs;
   const int n = c->nstate;
   // S = 2 Re C0^T C0 - Re c0(0) Re c0(0)^T  (DSYRK + DGER, wfn_initialize.f90:481-482)
   const bool sl = use_slice(c);
+  const G0Term g0 = g0_term(c, c->d_c0, c->d_c0);
   if (sl) {
     sg_slice(c, c->d_c0, c->d_plA, c->d_sgA);
-    sg_tn(c, c->tm_a_tn, c->tm_a_tn, 1, c->d_sgA, c->d_sgA, 2.0, c->d_gam);
+    sg_tn(c, c->tm_a_tn, c->tm_a_tn, 1, c->d_sgA, c->d_sgA, 2.0, c->d_gam, n, n, g0);
   } else {
-    RC(dg_tn(c, c->d_c0, n, c->d_c0, n, 2.0, c->d_gam, n, true));
+    RC(dg_tn(c, c->d_c0, n, c->d_c0, n, 2.0, c->d_gam, n, true, g0));
   }
-  ++c->nlaunch;
-  k_g0_correct<<<dim3(nblk(n), n), NTHR, 0, c->st>>>(n, h.ngpw, c->d_c0, c->d_c0, c->d_gam, c->d_occ, 0, 1);
   spin_mask(c, c->d_gam);
   if (n <= CHOL_NMAX) {
     const int np = (n + CHOL_B - 1) / CHOL_B * CHOL_B;
@@ -1276,7 +1282,14 @@ static int do_ortho(amdk_ctx *c, bool check = true, bool swap = true) {
   } else {
     RC(chol_inv_blocked(c, n));
   }
-  CK(cudaMemcpyAsync(c->h_info, c->d_info, 2 * sizeof(int), cudaMemcpyDeviceToHost, c->st));
+  // the status goes to the host beside the rotation (inside an iteration, on the side stream)
+  const bool aside = !check && c->overlap;
+  if (aside) {
+    CK(cudaEventRecord(c->ev_fork, c->st));
+    CK(cudaStreamWaitEvent(c->st2, c->ev_fork, 0));
+  }
+  CK(cudaMemcpyAsync(c->h_info, c->d_info, 2 * sizeof(int), cudaMemcpyDeviceToHost, aside ? c->st2 : c->st));
+  if (aside) CK(cudaEventRecord(c->ev_side_done, c->st2));
   if (check) {
     CK(cudaStreamSynchronize(c->st));
     RC(check_ortho(c));
@@ -1286,9 +1299,8 @@ static int do_ortho(amdk_ctx *c, bool check = true, bool swap = true) {
   if (sl)
     sg_nn(c, c->d_uinv, c->d_cp, 0, true);
   else
-    RC(dg_nn(c, c->d_c0, n, c->d_uinv, n, 1.0, 0.0, true, c->d_cp));
-  ++c->nlaunch;
-  k_zclean<<<nblk(n), NTHR, 0, c->st>>>(n, h.ngpw, c->d_cp);
+    RC(dg_nn(c, c->d_c0, n, c->d_uinv, n, 1.0, 0.0, true, c->d_cp, false, true));
+  if (aside) CK(cudaStreamWaitEvent(c->st, c->ev_side_done, 0));
   if (swap) std::swap(c->d_c0, c->d_cp);
   // the buffer whose digit planes d_plA holds (set again after a replayed graph)
   c->sg_c0_buf = sl ? (void *)(swap ? c->d_c0 : c->d_cp) : nullptr;
@@ -1555,7 +1567,6 @@ static int build_device(amdk_ctx *c) {
   RC(c->alloc(&c->d_vg, h.ngrho));
   RC(c->alloc(&c->d_vxg, h.ngrho));
   RC(c->alloc(&c->d_fp, 2L * h.ngrho));
-  RC(c->alloc(&c->d_fm, 2L * h.ngrho));
   RC(c->alloc(&c->d_gam, (size_t)h.nstate * h.nstate));
   RC(c->alloc(&c->d_uinv, (size_t)h.nstate * h.nstate));
   RC(c->alloc(&c->d_info, 2));  // [0] Cholesky status, [1] slice-GEMM wait status
@@ -1805,19 +1816,19 @@ template <typename C> static int seg_a_overlap(amdk_ctx *c) {
   CK(cudaStreamWaitEvent(c->st2, c->ev_fork, 0));
   {
     OnSideStream side(c);
+    RC(copy_istep(c));
     RC(energy_c0_terms(c));
     CK(cudaEventRecord(c->ev_side_done, c->st));
   }
   RC(density_pairs_t<C>(c));
-  RC(rhor2g_t<C>(c));
-  RC(potential_t<C>(c));
+  RC(grid_to_rays<C>(c, 1, nullptr, c->d_rho));
+  RC(potential_t<C>(c, true));
   CK(cudaStreamWaitEvent(c->st, c->ev_side_done, 0));
-  CK(cudaMemcpyAsync(c->h_pin, c->d_scal, sizeof(double) * S_NSCAL, cudaMemcpyDeviceToHost, c->st));
   pencil_vpsi<C>(c, T);
   xt_fwd<C>(c, T);
   RC(unpack_h<C>(c, 0, T, c->d_postp, c->d_postm, pencil_stride(c)));
   RC(do_gradient(c));
-  CK(cudaMemcpyAsync(c->h_pin + S_NSCAL, c->d_scal + S_GMAX, sizeof(double), cudaMemcpyDeviceToHost, c->st));
+  CK(cudaMemcpyAsync(c->h_pin, c->d_scal, sizeof(double) * S_NSCAL, cudaMemcpyDeviceToHost, c->st));
   return 0;
 }
 
@@ -1881,12 +1892,14 @@ static bool iter_overlap(const amdk_ctx *c) {
 static int seg_a_body(amdk_ctx *c) {
   const int q = (c->precision == AMDK_MIXED) ? 1 : 0;
   if (iter_overlap(c)) return q ? seg_a_overlap<float2>(c) : seg_a_overlap<double2>(c);
+  RC(copy_istep(c));
   RC(do_density(c));
   RC(do_potential(c));
-  RC(do_energy(c, nullptr));  // energies read after the end-of-iteration sync
+  RC(energy_c0_terms(c));
   RC(do_apply_h(c));
   RC(do_gradient(c));
-  CK(cudaMemcpyAsync(c->h_pin + S_NSCAL, c->d_scal + S_GMAX, sizeof(double), cudaMemcpyDeviceToHost, c->st));
+  // GEMAX and the energies, read after the segment's sync
+  CK(cudaMemcpyAsync(c->h_pin, c->d_scal, sizeof(double) * S_NSCAL, cudaMemcpyDeviceToHost, c->st));
   return 0;
 }
 static std::array<int, 4> seg_a_key(const amdk_ctx *c) {
@@ -1897,19 +1910,18 @@ static std::array<int, 4> seg_a_key(const amdk_ctx *c) {
 }
 // after segment A has finished: GEMAX, CHK_TFOR (gradient.f90:113-136)
 static int chk_tfor(amdk_ctx *c, int istep, double gcut, double *gm) {
-  *gm = c->h_pin[S_NSCAL];
+  *gm = c->h_pin[S_GMAX];
   if (!std::isfinite(*gm)) {
     set_error("non-finite wavefunction gradient");
     return AMDK_ERR_NONFINITE;
   }
   if (istep == 1) c->tfor = false;
   else if (*gm < 3 * gcut) c->tfor = true;
-  c->h_pin[S_NSCAL + 1] = (double)istep;  // read by the PCG step through a captured copy
   return 0;
 }
-static int seg_b_body(amdk_ctx *c, int istep) {
+static int seg_b_body(amdk_ctx *c) {
   if (c->tfor) RC(do_ionic_forces(c));
-  RC(do_pcg(c, istep));
+  RC(do_pcg(c));
   RC(do_ortho(c, false, false));
   return 0;
 }
@@ -2481,7 +2493,11 @@ int amdk_gradient(amdk_ctx *c, double *gemax) {
 int amdk_pcg(amdk_ctx *c, int istep) {
   if (!c || istep < 1) return AMDK_ERR_BADARG;
   cudaSetDevice(c->device);
-  return do_pcg(c, istep, true);
+  CK(cudaStreamSynchronize(c->st));  // an earlier copy of the step number may still read the pinned slot
+  c->h_pin[S_NSCAL + 1] = (double)istep;
+  RC(copy_istep(c));
+  gmax_precon(c);  // the caller may have changed C2 since the gradient
+  return do_pcg(c);
 }
 
 int amdk_scf_iteration(amdk_ctx *c, int istep, double gcut, amdk_energies *e, double *gemax, int *converged) {
@@ -2491,6 +2507,7 @@ int amdk_scf_iteration(amdk_ctx *c, int istep, double gcut, amdk_energies *e, do
   // graphs from the second iteration on, once this precision has run eagerly
   // (first-call setup of kernels and cuBLAS stays out of the capture)
   const bool graph = c->use_graphs && istep > 1 && c->warm[q];
+  c->h_pin[S_NSCAL + 1] = (double)istep;  // copied by segment A; nothing of this context is in flight
   cudaEventRecord(c->ev0, c->st);
   auto seg_a = [&]() -> int { return seg_a_body(c); };
   if (graph) RC(run_segment(c, seg_a_key(c), seg_a));
@@ -2500,7 +2517,7 @@ int amdk_scf_iteration(amdk_ctx *c, int istep, double gcut, amdk_energies *e, do
   CK(cudaStreamSynchronize(c->st));
   double gm = 0;
   RC(chk_tfor(c, istep, gcut, &gm));
-  auto seg_b = [&]() -> int { return seg_b_body(c, istep); };
+  auto seg_b = [&]() -> int { return seg_b_body(c); };
   if (graph) RC(run_segment(c, seg_b_key(c), seg_b));
   else RC(seg_b());
   cudaEventRecord(c->ev1, c->st);
@@ -2577,12 +2594,12 @@ int amdk_ensemble_iteration(amdk_ensemble *E, const int *istep, double gcut, amd
   }
   std::vector<std::array<int, 4>> keys(n);
   std::vector<amdk_ctx::SegGraph *> sgs(n);
-  auto run_all = [&](bool b, const std::vector<int> &steps) -> int {
+  auto run_all = [&](bool b) -> int {
     for (int i = 0; i < n; ++i) {
       amdk_ctx *c = E->m[i];
       keys[i] = b ? seg_b_key(c) : seg_a_key(c);
-      const int st = steps[i];
-      sgs[i] = b ? ensure_segment(c, keys[i], [&]() -> int { return seg_b_body(c, st); })
+      if (!b) c->h_pin[S_NSCAL + 1] = (double)istep[i];
+      sgs[i] = b ? ensure_segment(c, keys[i], [&]() -> int { return seg_b_body(c); })
                  : ensure_segment(c, keys[i], [&]() -> int { return seg_a_body(c); });
       if (!sgs[i]) {
         set_error("amdk_ensemble_iteration: a member's segment could not be captured");
@@ -2595,13 +2612,12 @@ int amdk_ensemble_iteration(amdk_ensemble *E, const int *istep, double gcut, amd
     for (int i = 0; i < n; ++i) account_segment(E->m[i], *sgs[i]);
     return 0;
   };
-  const std::vector<int> steps(istep, istep + n);
   CK(cudaEventRecord(E->ev0, E->st));
-  RC(run_all(false, steps));
+  RC(run_all(false));
   CK(cudaStreamSynchronize(E->st));
   std::vector<double> gm(n);
   for (int i = 0; i < n; ++i) RC(chk_tfor(E->m[i], istep[i], gcut, &gm[i]));
-  RC(run_all(true, steps));
+  RC(run_all(true));
   CK(cudaEventRecord(E->ev1, E->st));
   CK(cudaEventSynchronize(E->ev1));
   float ms = 0;
@@ -2665,9 +2681,7 @@ int amdk_wfn_extrapolate(amdk_ctx *c) {
       const double2 *hj = c->d_hist[j - 1];
       // M = 2 Re C_j^T C0 - Re c_j(0) Re c0(0)^T aligns step j's occupied
       // subspace with the current one; cp (+)= w_j C_j M
-      RC(dg_tn(c, hj, n, c->d_c0, n, 2.0, c->d_gam, n));
-      ++c->nlaunch;
-      k_g0_correct<<<dim3(nblk(n), n), NTHR, 0, c->st>>>(n, h.ngpw, hj, c->d_c0, c->d_gam, c->d_occ, 0, 0);
+      RC(dg_tn(c, hj, n, c->d_c0, n, 2.0, c->d_gam, n, false, g0_term(c, hj, c->d_c0)));
       spin_mask(c, c->d_gam);
       RC(dg_nn(c, hj, n, c->d_gam, n, w[j], j == 1 ? 0.0 : 1.0, false, c->d_cp));
     }
@@ -2764,9 +2778,7 @@ int amdk_fft_sphere(amdk_ctx *c, int sign, double *coef, double *grid) {
   long npt = (long)h.nr[0] * h.nr[1] * h.nr[2];
   if (sign == -1) {
     CK(cudaMemcpyAsync(c->d_vxg, coef, sizeof(double2) * h.ngrho, cudaMemcpyHostToDevice, c->st));
-    ++c->nlaunch;
-    k_conj_field<<<nblk(h.ngrho), NTHR, 0, c->st>>>(h.ngrho, c->d_vxg, c->d_fm);
-    RC(field_to_grid(c, 1, c->d_vxg, c->d_fm, c->d_cgrid));
+    RC(field_to_grid(c, 1, c->d_vxg, c->d_cgrid));
     CK(cudaMemcpyAsync(grid, c->d_cgrid, sizeof(double2) * npt, cudaMemcpyDeviceToHost, c->st));
   } else {
     CK(cudaMemcpyAsync(c->d_cgrid, grid, sizeof(double2) * npt, cudaMemcpyHostToDevice, c->st));
@@ -2831,7 +2843,8 @@ static int noalloc_scratch(unsigned char **out) {
   return 0;
 }
 
-// Scratch bytes one transform of this context's density sphere needs.
+// Scratch bytes one transform of this context's density sphere needs (with the
+// field of -G values that the limit on the grid size has always counted).
 static size_t noalloc_bytes(amdk_ctx *c, size_t *rbytes, size_t *sbytes) {
   auto round256 = [](size_t b) { return (b + 255) & ~(size_t)255; };
   *rbytes = round256((size_t)rstride(c, 1) * sizeof(double2));
@@ -2861,13 +2874,10 @@ int amdk_fft_sphere_noalloc(amdk_ctx *c, int sign, double *coef, double *grid) {
   // for all work on the device before reading them
   CK(cudaDeviceSynchronize());
   const XBufs b{base, base + rbytes};
-  double2 *FM = (double2 *)(base + rbytes + sbytes);
   const long npt = (long)h.nr[0] * h.nr[1] * h.nr[2];
   if (sign == -1) {
     // coef (+G half) -> complex grid; the -G values are conj(coef)
-    ++c->nlaunch;
-    k_conj_field<<<nblk(h.ngrho), NTHR, 0, c->st>>>(h.ngrho, (const double2 *)coef, FM);
-    RC(field_to_grid<double2>(c, 1, (const double2 *)coef, FM, (double2 *)grid, b));
+    RC(field_to_grid<double2>(c, 1, (const double2 *)coef, (double2 *)grid, b));
   } else {
     // complex grid -> coef = F(+G)/N
     RC(grid_to_rays<double2>(c, 1, (const double2 *)grid, nullptr, b));
@@ -3013,12 +3023,13 @@ int amdk_slab_gram(amdk_slab *s, const double *a, const double *b, int n, double
     return 0;
   }
   // the FP64 tensor-core product over the rank's 2 ngpw_local real components
-  RC(dg_tn(c, a, n, b, n, 2.0, out, n, a == b, 2L * s->ng, st));
+  G0Term g0;
   if (s->gzero == 0) {  // the rank holding G = 0 (local index 0) removes its doubled term
-    ++c->nlaunch;
-    k_g0_correct<<<dim3(nblk(n), n), NTHR, 0, st>>>(n, s->ng, (const double2 *)a, (const double2 *)b, out, c->d_occ, 0,
-                                                    0);
+    g0.a = a;
+    g0.b = b;
+    g0.ld = 2L * s->ng;
   }
+  RC(dg_tn(c, a, n, b, n, 2.0, out, n, a == b, g0, 2L * s->ng, st));
   CK(cudaGetLastError());
   int expired = 0;
   CK(cudaMemcpyAsync(&expired, c->d_info + 1, sizeof(int), cudaMemcpyDeviceToHost, st));

@@ -225,7 +225,8 @@ __global__ void __launch_bounds__(DG_THREADS, 3) k_dgemm_tn(const __grid_constan
 // With sym, an element of a tile above the diagonal is written at (i, j) and
 // (j, i).
 __global__ void __launch_bounds__(256) k_dgemm_tn_sum(const double *part, int nb, int seg, int ntile, int ktiles, int mt,
-                                                      int sym, int m, int n, double alpha, double *out, int ldo) {
+                                                      int sym, int m, int n, double alpha, double *out, int ldo,
+                                                      G0Term g0) {
   __shared__ double red[8][32];
   const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
   const long tot = (long)ntile * (DG_T * DG_T), U = (long)ntile * ktiles;
@@ -260,8 +261,8 @@ __global__ void __launch_bounds__(256) k_dgemm_tn_sum(const double *part, int nb
       double v = red[0][lane];
 #pragma unroll
       for (int k = 1; k < 8; ++k) v += red[k][lane];
-      out[i + (long)ldo * j] = alpha * v;
-      if (sym && it != jt) out[j + (long)ldo * i] = alpha * v;
+      out[i + (long)ldo * j] = g0(alpha * v, i, j);
+      if (sym && it != jt) out[j + (long)ldo * i] = g0(alpha * v, j, i);
     }
     __syncthreads();
   }
@@ -273,7 +274,8 @@ __global__ void __launch_bounds__(256) k_dgemm_tn_sum(const double *part, int nb
 // G is upper triangular (its lower part holds zeros) and the products with the
 // lower part are skipped 16 columns at a time.  With g0twice the product's
 // rows 0 and 1 (G = 0 of a projector matrix that holds half its value there)
-// count twice.
+// count twice; with zclean row 1 of out, Im c(G=0), is set to zero (ZCLEAN,
+// wfn_initialize.f90:531-558).
 // A warp's MMAs take the columns j as the M index and the long index r as N,
 // with the n index of two adjacent N tiles interleaved (r = 2n, 2n + 1), so
 // that a lane reads 16 bytes of every operand at a time, free of bank
@@ -289,7 +291,7 @@ __global__ void __launch_bounds__(256) k_dgemm_tn_sum(const double *part, int nb
 __global__ void __launch_bounds__(DG_NN_THREADS, 2) k_dgemm_nn(const __grid_constant__ CUtensorMap ta,
                                                                const __grid_constant__ CUtensorMap tg, long K, int n1,
                                                                int n, double alpha, double beta, int upper,
-                                                               int g0twice, double *out, long ldo, int *err,
+                                                               int g0twice, int zclean, double *out, long ldo, int *err,
                                                                long plim) {
   extern __shared__ unsigned char dg_raw[];
   unsigned char *sm = dg_align1k(dg_raw);
@@ -422,6 +424,7 @@ __global__ void __launch_bounds__(DG_NN_THREADS, 2) k_dgemm_nn(const __grid_cons
             const double f = g0twice && r0 + 16 * p + e == 0 ? 2.0 * alpha : alpha;
             double2 v = make_double2(f * acc[m][p][0][2 * h + e] + beta * old[h][p][e].x,
                                      f * acc[m][p][1][2 * h + e] + beta * old[h][p][e].y);
+            if (zclean && r0 + 16 * p + e == 0) v.y = 0.0;
             if (bad) v.x = v.y = __longlong_as_double(0x7ff8000000000000LL);
             *reinterpret_cast<double2 *>(o + ldo * (8 * h) + 16 * p + 2 * e) = v;
           }

@@ -493,10 +493,14 @@ __global__ void __launch_bounds__(256) k_x_bwd_pair(const double2 *__restrict__ 
   }
 }
 
-// Backward X pass from a G field given at +G (fp) and -G (fm), t-th field at
-// fp + t*ngrho (eval_pot / rhog2r / GRAD_CAL packs).
-template <typename C, int N = 0>
-__global__ void __launch_bounds__(256) k_x_bwd_field(const double2 *__restrict__ fp, const double2 *__restrict__ fm, int ngmax,
+// Backward X pass of real fields given at +G (-G: the conjugate), the t-th
+// field at f + t*ngmax (FS_REAL), or of the packed fields rho + i d_x rho
+// (t = 0) and d_y rho + i d_z rho (t = 1) of GRAD_CAL (xc.f90:471-487), formed
+// from rho(G) = f and G as they are gathered (FS_GRAD).
+enum { FS_REAL = 0, FS_GRAD = 1 };
+template <typename C, int N, int SRC>
+__global__ void __launch_bounds__(256) k_x_bwd_field(const double2 *__restrict__ f, const double *__restrict__ gvec,
+                                                     double tpiba, int ngmax,
                                                      int sphere, int T, Geom g, Plan<C> p, C *__restrict__ rb) {
   extern __shared__ unsigned char smraw[];
   C *sa = reinterpret_cast<C *>(smraw);
@@ -516,7 +520,19 @@ __global__ void __launch_bounds__(256) k_x_bwd_field(const double2 *__restrict__
       const int code = g.gmap[(long)r * n1 + k];
       const int ig = (code > 0 ? code : -code) - 1;
       if (code != 0 && ig < ngmax) {
-        double2 a = (code > 0) ? fp[(long)t * ngmax + ig] : fm[(long)t * ngmax + ig];
+        const double sg = code > 0 ? 1.0 : -1.0;
+        double2 a = f[(SRC == FS_REAL ? (long)t * ngmax : 0L) + ig];
+        a.y *= sg;
+        if (SRC == FS_GRAD) {
+          // f + i (i G_x f) and i G_y f + i (i G_z f), of f(G) or its conjugate at -G
+          if (t == 0) {
+            const double gx = sg * (tpiba * gvec[3 * ig]);
+            a = make_double2(a.x - gx * a.x, a.y - gx * a.y);
+          } else {
+            const double ax = -(sg * tpiba) * gvec[3 * ig + 2], ay = (sg * tpiba) * gvec[3 * ig + 1];
+            a = make_double2(ax * a.x - ay * a.y, ax * a.y + ay * a.x);
+          }
+        }
         v = mk((decltype(v.x))a.x, (decltype(v.x))a.y);
       }
     }

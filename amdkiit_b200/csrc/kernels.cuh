@@ -90,7 +90,7 @@ __device__ void reduce_and_finish(const double (&v)[NK], double *part, double *o
 // slots of the device scalar array: CG norms, energy sums, GEMAX, CG step
 enum { S_GGPREV = 1, S_EH = 2, S_ELOC, S_EXC, S_EKIN, S_ENL, S_ISTEP = 8, S_GMAX = 9, S_GG = 10, S_NSCAL = 16 };
 // tickets of the self-finishing reductions (one per kernel)
-enum { TK_VLOC = 0, TK_XC, TK_ENL, TK_EKIN, TK_GRAD, TK_N = 8 };
+enum { TK_VLOC = 0, TK_XC, TK_ENL, TK_EKIN, TK_GRAD, TK_PCG, TK_N = 8 };
 
 // ---------------------------------------------------------------- tables
 // spline_inter (spline_inter.f90:1-36) evaluated at one point; the hunt is
@@ -239,15 +239,25 @@ __global__ void k_gather_p(int ng, const int *pos_p, const C *rb, double scale, 
   out[g] = make_double2((double)v.x * scale, (double)v.y * scale);
 }
 
-// eval_pot (potential.f90:4-46) in G space + e_hartree / pp_energy E_loc
-// partial sums: part[0*nb+b] = Re sum 4pi/G^2 |rho+rho_ion|^2,
+// eval_pot (potential.f90:4-46) in G space + e_hartree / pp_energy E_loc, with
+// GATHER from the forward transform of rho in the ray buffer (rhor2g's last
+// step: rho(G) = F(+G)/N is stored as well); partial sums: part[0*nb+b] = Re sum 4pi/G^2 |rho+rho_ion|^2,
 // part[1*nb+b] = Re sum eigrxvps conj(rho) (G=0 weighted 1/2).
-__global__ void k_vloc_g(int ngrho, const double *hg, double tpiba2, const double2 *rhog, const double2 *erhos,
+template <typename C, bool GATHER>
+__global__ void k_vloc_g(int ngrho, const int *pos_p, const C *rb, double scale, const double *hg, double tpiba2,
+                         double2 *rhog, const double2 *erhos,
                          const double2 *evps, double2 *vg, double *part, double *out, unsigned *ticket) {
   const double fp = 16.0 * atan(1.0);
   double eh = 0, el = 0;
   for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ngrho; g += gridDim.x * blockDim.x) {
-    double2 rg = rhog[g], e = evps[g];
+    double2 rg, e = evps[g];
+    if (GATHER) {
+      const C v = rb[pos_p[g]];
+      rg = make_double2((double)v.x * scale, (double)v.y * scale);
+      rhog[g] = rg;
+    } else {
+      rg = rhog[g];
+    }
     if (g == 0) {
       vg[0] = make_double2(0.0, 0.0);
       el += 0.5 * (e.x * rg.x + e.y * rg.y);
@@ -261,26 +271,6 @@ __global__ void k_vloc_g(int ngrho, const double *hg, double tpiba2, const doubl
   }
   const double v[2] = {eh, el};
   reduce_and_finish<2>(v, part, out, ticket);  // out[0] = E_H sum, out[1] = E_loc sum
-}
-
-// GRAD_CAL fields (xc.f90:471-487): t=0: rho + i d_x rho, t=1: d_y rho + i d_z rho
-__global__ void k_grad_fields(int ngrho, const double *gvec, double tpiba, const double2 *rhog, double2 *fp, double2 *fm) {
-  int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= ngrho) return;
-  double2 r = rhog[g];
-  double gx = tpiba * gvec[3 * g], gy = gvec[3 * g + 1], gz = gvec[3 * g + 2];
-  fp[g] = make_double2(r.x - gx * r.x, r.y - gx * r.y);
-  fm[g] = make_double2(r.x + gx * r.x, -(r.y + gx * r.y));
-  // tpiba (i gy - gz) r  and tpiba (-i gy + gz) conj(r)
-  double ax = -tpiba * gz, ay = tpiba * gy;
-  fp[ngrho + g] = make_double2(ax * r.x - ay * r.y, ax * r.y + ay * r.x);
-  double bx = tpiba * gz, by = -tpiba * gy;
-  fm[ngrho + g] = make_double2(bx * r.x + by * r.y, by * r.x - bx * r.y);
-}
-__global__ void k_conj_field(int ng, const double2 *fp, double2 *fm) {
-  int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= ng) return;
-  fm[g] = make_double2(fp[g].x, -fp[g].y);
 }
 
 // ---------------------------------------------------------------- XC
@@ -725,22 +715,6 @@ inline void aspc_coefficients(int npoints, double *w) {
   const double den = binom(2 * K + 2, K + 1);
   for (int j = 1; j <= npoints; ++j) w[j - 1] = ((j & 1) ? 1.0 : -1.0) * j * binom(2 * K + 4, K + 2 - j) / den;
 }
-// rank-1 G=0 correction and occupation mask of OVLAP_D / ortho_gs DGER
-// (wfn_initialize.f90:257,482): A(i,j) -= Re a_i(0) Re b_j(0); mask fsc
-__global__ void k_g0_correct(int n, int ngpw, const double2 *a, const double2 *b, double *A, const double *occ, int mask,
-                             int upper_only) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
-  if (i >= n || j >= n) return;
-  if (upper_only && i > j) return;
-  double v = A[i + (long)n * j] - a[(long)i * ngpw].x * b[(long)j * ngpw].x;
-  if (mask) v *= (occ[i] == 0.0 ? 0.0 : 1.0) * (occ[j] == 0.0 ? 0.0 : 1.0);
-  A[i + (long)n * j] = v;
-}
-// ZCLEAN (wfn_initialize.f90:531-558)
-__global__ void k_zclean(int n, int ngpw, double2 *c) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) c[(long)i * ngpw].y = 0.0;
-}
 // eval_GMAX (gradient.f90:36-61) and the preconditioned-gradient norm of
 // PRECON + GGNORM (cg.f90:102-107, 281-311) in one pass over the occupied
 // bands of C2: out[0] = GEMAX = max |C2|, out[1] = sum_i DOTP(cp_i, cp_i)
@@ -782,11 +756,21 @@ __global__ void k_gmax_precon(int ngpw, int nocc, const double *vpp, const doubl
 }
 // PCG direction and step (cg.f90:109-143) with cp = f_i^-1 K(G) C2 (PRECON,
 // cg.f90:281-311); gamma = forget * ggnorm(new) / ggnorm(previous)
-__global__ void k_pcg_update(int ngpw, int nstate, const double *scal, const double *vpp, const double *occ,
+// The last block to have read the scalars makes the norm the previous one.
+__global__ void k_pcg_update(int ngpw, int nstate, double *scal, unsigned *ticket, const double *vpp, const double *occ,
                              const double2 *__restrict__ c2, double2 *__restrict__ hnm1, double2 *__restrict__ c0) {
   const int istep = (int)scal[S_ISTEP];
   const double forget = istep <= 10 ? 0.60 : (istep <= 20 ? 0.91 : 0.95);
-  const double gamma = (istep == 1) ? 0.0 : forget * (scal[S_GG] / scal[S_GGPREV]);
+  const double gg = scal[S_GG];
+  const double gamma = (istep == 1) ? 0.0 : forget * (gg / scal[S_GGPREV]);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(ticket, 1u) == gridDim.x - 1) {
+      scal[S_GGPREV] = gg;
+      *ticket = 0u;
+    }
+  }
   const double dt = 5.0 * 5.0 / 400.0;
   BandWalk w((long)ngpw * nstate, ngpw);
   int bf = -1;
@@ -812,7 +796,6 @@ __global__ void k_pcg_update(int ngpw, int nstate, const double *scal, const dou
     c0[w.k] = x;
   }
 }
-__global__ void k_copy_scalar(const double *src, double *dst) { *dst = *src; }
 
 // Shared-memory blocked Cholesky + inverse for n <= CHOL_NMAX, one block of
 // CHOL_NT threads (DPOTRF + DTRTRI of UINV, wfn_initialize.f90:504-530).

@@ -777,6 +777,31 @@ __global__ void k_v_permute(int n, int nx, int n1f, int n2f, const double *__res
   }
 }
 
+// The same from the real part of a complex grid, which is stored in v as well
+template <typename Rl>
+__global__ void k_v_store(int n, int n1f, int n2f, const double2 *__restrict__ grid, double *__restrict__ v,
+                          Rl *__restrict__ vp) {
+  __shared__ double tile[32][33];
+  const int kp = blockIdx.z;
+  const int kz = perm_index(kp, n1f, n2f);
+  const int kx0 = blockIdx.x * 32, q0 = blockIdx.y * 32;
+  for (int j = threadIdx.y; j < 32; j += blockDim.y) {
+    const int q = q0 + j, kx = kx0 + threadIdx.x;
+    double x = 0.0;
+    if (kx < n && q < n) {
+      const long o = ((long)kz * n + perm_index(q, n1f, n2f)) * n + kx;
+      x = grid[o].x;
+      v[o] = x;
+    }
+    tile[j][threadIdx.x] = x;
+  }
+  __syncthreads();
+  for (int j = threadIdx.y; j < 32; j += blockDim.y) {
+    const int kx = kx0 + j, q = q0 + threadIdx.x;
+    if (kx < n && q < n) vp[((long)kx * n + kp) * n + q] = (Rl)tile[threadIdx.x][j];
+  }
+}
+
 // Slab decomposition: the +G / -G positions of a rank's G vectors in its
 // send/return buffer [kx][t][local ray] for T pairs (row = T * local rays),
 // from the planes and local rays of the two positions

@@ -47,6 +47,21 @@
 
 namespace amdk {
 
+// The G = 0 term of a band-space matrix and its occupation mask (OVLAP_D,
+// wfn_initialize.f90:257; the DGER of ortho_gs, :482), applied where the
+// product is written: A(i,j) -= Re a_i(0) Re b_j(0), zero between bands of zero
+// occupation where occ is given.  a, b: real views, ld reals per band; a null: none.
+struct G0Term {
+  const double *a = nullptr, *b = nullptr, *occ = nullptr;
+  long ld = 0;
+  __device__ __forceinline__ double operator()(double v, int i, int j) const {
+    if (!a) return v;
+    v -= a[(long)i * ld] * b[(long)j * ld];
+    if (occ) v *= (occ[i] == 0.0 ? 0.0 : 1.0) * (occ[j] == 0.0 ? 0.0 : 1.0);
+    return v;
+  }
+};
+
 constexpr int SG_S = 4;          // digit planes per operand
 constexpr int SG_M = 128;        // rows per plane (bands, padded)
 constexpr int SG_TN_KT = 64;     // k bytes per TN stage (64-byte swizzle)
@@ -433,7 +448,7 @@ __global__ void __launch_bounds__(SG_RG * SG_M) k_sgemm_reduce(int nchunk, const
                                                                const double *__restrict__ sa,
                                                                const double *__restrict__ sb,
                                                                const double *__restrict__ nsq, double alpha,
-                                                               double *__restrict__ out, int ldo) {
+                                                               double *__restrict__ out, int ldo, G0Term g0) {
   const int m = threadIdx.x % SG_M, g = threadIdx.x / SG_M, n = blockIdx.x;
   __shared__ double red[SG_RG][SG_M];
   double s = 0.0;
@@ -451,7 +466,7 @@ __global__ void __launch_bounds__(SG_RG * SG_M) k_sgemm_reduce(int nchunk, const
       for (int i = 0; i < SG_SEG; ++i) q += nsq[m * SG_SEG + i];
       v = alpha * q;
     }
-    out[m + (long)ldo * n] = v;
+    out[m + (long)ldo * n] = g0(v, m, n);
   }
 }
 
@@ -470,7 +485,8 @@ template <int S> struct SgNn {
 // accumulators, which are combined exactly in 64-bit integers
 // (sum_d acc_d 128^{S-1-d}, below 2^45) and converted once; the old values of
 // a subtraction are loaded before the accumulators are read.  MODE 0 stores,
-// 1 subtracts, 2 stores and also cuts the result into the S digit planes
+// 1 subtracts (setting real index 1, Im c(G=0), to zero as ZCLEAN does), 2
+// stores and also cuts the result into the S digit planes
 // dig[t][n][m] with the fixed scale sigma = 2 (an orthonormalisation: its
 // output bands satisfy |x| <= 1), ready as the next product's operand,
 // setting its real index 1 (Im c(G=0)) to zero as ZCLEAN does.
@@ -592,7 +608,7 @@ __global__ void __launch_bounds__(SG_NN_THREADS, 1) k_sgemm_nn(const __grid_cons
           for (int j = 0; j < 8; ++j) {
             const int n = 8 * cb + j;
             double val = v[j];
-            if (MODE == 1) val = old[j] - val;
+            if (MODE == 1) val = (gm == 1) ? 0.0 : old[j] - val;
             if (MODE == 2) {
               val = (gm == 1) ? 0.0 : val;
               int dd[S];
