@@ -816,54 +816,75 @@ __global__ void k_pcg_update(int ngpw, int nstate, double *scal, unsigned *ticke
 constexpr int CHOL_NMAX = 144;
 constexpr int CHOL_NT = 512;
 constexpr int CHOL_B = 16;
+// 1/sqrt(d) for d > 0: the hardware's approximation and two Newton steps
+// y += y (1 - d y^2) / 2, straight-line code (the library call's branch keeps the
+// scheduler from running the previous step's updates under it); tiny d scaled
+__device__ __forceinline__ double chol_rsqrt(double d) {
+  const bool tiny = d < 0x1p-900;
+  const double x = tiny ? d * 0x1p600 : d;
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+#pragma unroll
+  for (int it = 0; it < 2; ++it) y = fma(0.5 * y, fma(-x * y, y, 1.0), y);
+  return tiny ? y * 0x1p300 : y;
+}
+// Factor and invert one 16 x 16 diagonal block by a warp: forward elimination of
+// [S | 1] gives [U | U^-T], lane l < 16 holding column l of S and lane 16 + c
+// column c of the identity, so the inverse costs no step of its own (row i of
+// X = U^-1 ends in lane 16 + i).
 __device__ __forceinline__ void warp_chol_inv16(double *D, int ld, int base, int *bad) {
   const int l = threadIdx.x & 31;
-  const bool own = l < CHOL_B;
-  double col[CHOL_B], invd[CHOL_B];  // invd[j] = 1 / U_jj, the same in every lane
+  double col[CHOL_B];
   int badj = 0;
 #pragma unroll
-  for (int r = 0; r < CHOL_B; ++r) col[r] = own ? D[r + ld * l] : 0.0;
+  for (int r = 0; r < CHOL_B; ++r) col[r] = l < CHOL_B ? (r <= l ? D[r + ld * l] : 0.0) : (r == l - CHOL_B ? 1.0 : 0.0);
 #pragma unroll
   for (int j = 0; j < CHOL_B; ++j) {
     const double d = __shfl_sync(0xffffffffu, col[j], j);
     if (!(d > 0.0) && badj == 0) badj = base + j + 1;
-    const double inv = rsqrt(d);
-    invd[j] = inv;
-    if (l == j) col[j] = d * inv;
-    else if (l > j) col[j] *= inv;
-    // constant bounds: the loop unrolls and col[] stays in registers (a bound
-    // that depends on j left it in local memory, doubling the kernel's time)
+    col[j] *= chol_rsqrt(d);
+    // constant bounds: the loop unrolls and col[] stays in registers; the next
+    // pivot's row is updated first.  Lanes below the row hold nothing that is
+    // read again, so every lane takes part.
 #pragma unroll
-    for (int a = 0; a < CHOL_B; ++a) {
-      if (a > j) {
-        const double uja = __shfl_sync(0xffffffffu, col[j], a);
-        if (l >= a) col[a] -= uja * col[j];
-      }
+    for (int a = j + 1; a < CHOL_B; ++a) {
+      const double uja = __shfl_sync(0xffffffffu, col[j], a);
+      col[a] = fma(-uja, col[j], col[a]);
     }
   }
   if (l == 0 && badj && *bad == 0) *bad = badj;
-  if (own) {
+  __syncwarp();
+  if (l >= CHOL_B) {
+    const int i = l - CHOL_B;
 #pragma unroll
     for (int r = 0; r < CHOL_B; ++r)
-      if (r <= l) D[r + ld * l] = col[r];
+      if (r >= i) D[i + ld * r] = col[r];
   }
-  __syncwarp();
-  double x[CHOL_B];
+}
+// D (16 x 16) -= P^T P on the diagonal and above, P the 16 rows above D, by a
+// warp on the FP64 tensor cores (mma.m16n8k8: the A fragment of P^T is also the
+// B fragment of P)
+__device__ __forceinline__ void warp_syrk16(double *D, const double *P, int ld) {
+  const int l = threadIdx.x & 31, g = l >> 2, t = l & 3;
+  double acc[2][4] = {};
 #pragma unroll
-  for (int i = CHOL_B - 1; i >= 0; --i) {
-    double t = 0.0;
+  for (int kb = 0; kb < 2; ++kb) {
+    const double *q = P + 8 * kb + t + ld * g;
+    const double a0 = q[0], a1 = q[8 * ld], a2 = q[4], a3 = q[8 * ld + 4];
 #pragma unroll
-    for (int k = 0; k < CHOL_B; ++k)
-      if (k > i) t += D[i + ld * k] * x[k];
-    const double di = invd[i];
-    x[i] = (i == l) ? di : ((i < l) ? -t * di : 0.0);
+    for (int n = 0; n < 2; ++n)
+      asm volatile(
+          "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+          : "+d"(acc[n][0]), "+d"(acc[n][1]), "+d"(acc[n][2]), "+d"(acc[n][3])
+          : "d"(a0), "d"(a1), "d"(a2), "d"(a3), "d"(n ? a1 : a0), "d"(n ? a3 : a2));
   }
-  __syncwarp();
-  if (own) {
 #pragma unroll
-    for (int r = 0; r < CHOL_B; ++r)
-      if (r <= l) D[r + ld * l] = x[r];
-  }
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int r = g + 8 * (e >> 1), c = 8 * n + 2 * t + (e & 1);
+      if (r <= c) D[r + ld * c] -= acc[n][e];
+    }
 }
 
 // A (leading dimension lda) in, U^-1 into Ui (leading dimension ldu); a
@@ -916,18 +937,7 @@ __global__ void __launch_bounds__(CHOL_NT) k_chol_inv_s(int n, const double *A, 
       // lookahead: this step's update of the next diagonal block, then its
       // factor and inverse
       if (c0 < np) {
-        for (int e = lane; e < CHOL_B * CHOL_B; e += 32) {
-          const int r = c0 + (e & 15), c = c0 + (e >> 4);
-          if (r <= c) {
-            double t0 = 0.0, t1 = 0.0;
-#pragma unroll
-            for (int s = 0; s < CHOL_B; s += 2) {
-              t0 = fma(M[(k0 + s) + ld * r], M[(k0 + s) + ld * c], t0);
-              t1 = fma(M[(k0 + s + 1) + ld * r], M[(k0 + s + 1) + ld * c], t1);
-            }
-            M[r + ld * c] -= t0 + t1;
-          }
-        }
+        warp_syrk16(M + c0 + ld * c0, M + k0 + ld * c0, ld);
         __syncwarp();
         warp_chol_inv16(M + c0 + ld * c0, ld, c0, &bad);
       }
