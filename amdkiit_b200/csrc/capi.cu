@@ -88,7 +88,7 @@ struct amdk_ctx {
   Plan<double2> pd[3];
   Plan<float2> pf[3];
   std::vector<void *> allocs;
-  int *d_gmap = nullptr, *d_posp = nullptr, *d_posm = nullptr, *d_zlist[2] = {}, *d_rayidx[2] = {};
+  int *d_gmap = nullptr, *d_posp = nullptr, *d_posm = nullptr, *d_zlist[2] = {}, *d_rayidx[2] = {}, *d_zinv[2] = {};
   int *d_inyh = nullptr;
   double *d_hg = nullptr, *d_gvec = nullptr;
   long rb_elems_pw = 0, sb_elems_pw = 0, rb_elems_rho = 0, sb_elems_rho = 0;
@@ -314,6 +314,25 @@ template <auto K> static void smem_opt_in() {
   (void)done;
 }
 
+// the twiddle tables of a length, a kernel parameter
+template <typename C, int N> static const FftTw<C, N> &fft_tw() {
+  static const FftTw<C, N> t = []() {
+    FftTw<C, N> x{};
+    if constexpr (N > 0) {
+    constexpr int N1 = fft_n1(N), N2 = N / N1;
+    const double tp = 8.0 * std::atan(1.0);
+    for (int i = 0; i < N; ++i)
+      for (int h = 0; h < 2; ++h) {
+        const int d = h ? N2 : N1, e = (i / d) * (i % d) % N;
+        const double a = -tp * (double)e / (double)N;
+        x.t[h * N + i].x = (decltype(x.t[0].x))std::cos(a);
+        x.t[h * N + i].y = (decltype(x.t[0].x))std::sin(a);
+      }
+    }
+    return x;
+  }();
+  return t;
+}
 // shared memory of the slab-path kernels: two tiles and the twiddle tables (2n)
 template <typename C> static size_t x_smem(int n1) { return 2 * (size_t)n1 * (LX + 1) * sizeof(C) + 2 * n1 * sizeof(C); }
 template <typename C> static size_t yz_smem(int n) { return 2 * (size_t)n * TX * sizeof(C) + 2 * n * sizeof(C); }
@@ -321,11 +340,6 @@ template <typename C> static size_t yz_smem(int n) { return 2 * (size_t)n * TX *
 template <typename C> static void set_smem_attrs() {
   int mx = 227 * 1024;
   cudaFuncSetAttribute(k_x_bwd_pair<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_x_fwd<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_y<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_z<C, Z_TO_GRID>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_z<C, Z_FROM_GRID_REAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_z<C, Z_FROM_GRID_CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
   cudaFuncSetAttribute(k_z<C, Z_VPSI>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
   cudaFuncSetAttribute(k_z<C, Z_DENSITY>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
 }
@@ -357,15 +371,21 @@ template <typename C> static void y_pass(amdk_ctx *c, int sphere, int dir, int T
   ++c->nlaunch;
   with_n(g.n2, [&](auto NC) {
     constexpr int N = decltype(NC)::value;
-    smem_opt_in<k_y<C, N>>();
-    k_y<C, N><<<grid, NTHR, yz_smem<C>(g.n2), c->st>>>(sphere, dir, g, plan<C>(c, 1), (C *)rays_of(c, sphere, b),
-                                                      (C *)slab_of(c, b), rstride(c, sphere), sstride(c, sphere));
+    auto run = [&](auto K) {
+      K<<<grid, N > 0 ? direct_threads(N > 0 ? N : 36, TX) : NTHR, N > 0 ? (size_t)N * TX * sizeof(C) : yz_smem<C>(g.n2), c->st>>>(
+          sphere, g, plan<C>(c, 1), fft_tw<C, N>(), (C *)rays_of(c, sphere, b), (C *)slab_of(c, b), rstride(c, sphere),
+          sstride(c, sphere));
+    };
+    smem_opt_in<k_y<C, N, 1>>();
+    smem_opt_in<k_y<C, N, -1>>();
+    if (dir > 0) run(k_y<C, N, 1>);
+    else run(k_y<C, N, -1>);
   });
   prof_end(c);
 }
+// T transforms between the slab buffer and the grids cg (complex) or rg (real)
 template <typename C, int MODE>
-static void z_pass(amdk_ctx *c, int sphere, int T, double2 *cg, const double *rg, int pair0 = 0,
-                   const XBufs &b = XBufs{}) {
+static void z_pass(amdk_ctx *c, int sphere, int T, double2 *cg, double *rg, int pair0 = 0, const XBufs &b = XBufs{}) {
   const Geom &g = c->geom;
   dim3 grid((g.n1 + TX - 1) / TX, g.n2, MODE == Z_DENSITY ? 1 : T);
   long gs = (long)g.n1 * g.n2 * g.n3;
@@ -377,13 +397,28 @@ static void z_pass(amdk_ctx *c, int sphere, int T, double2 *cg, const double *rg
   ++c->nlaunch;
   with_n(g.n3, [&](auto NC) {
     constexpr int N = decltype(NC)::value;
-    smem_opt_in<k_z<C, MODE, N>>();
-    k_z<C, MODE, N><<<grid, NTHR, yz_smem<C>(g.n3), c->st>>>(sphere, T, g, plan<C>(c, 2), (C *)slab_of(c, b),
-                                                             sstride(c, sphere), cg, rg, gs, c->d_vpot, c->d_rho,
-                                                             c->d_wa + pair0, c->d_wb + pair0);
+    if constexpr (N > 0 && MODE != Z_VPSI && MODE != Z_DENSITY) {
+      smem_opt_in<k_z_field<C, MODE, N>>();
+      k_z_field<C, MODE, N><<<grid, direct_threads(N, TX), (size_t)N * TX * sizeof(C), c->st>>>(
+          sphere, g, fft_tw<C, N>(), (C *)slab_of(c, b), sstride(c, sphere), cg, rg, gs);
+    } else {
+      smem_opt_in<k_z<C, MODE, N>>();
+      k_z<C, MODE, N><<<grid, NTHR, yz_smem<C>(g.n3), c->st>>>(sphere, T, g, plan<C>(c, 2), (C *)slab_of(c, b),
+                                                               sstride(c, sphere), cg, rg, gs, c->d_vpot, c->d_rho,
+                                                               c->d_wa + pair0, c->d_wb + pair0);
+    }
   });
   prof_end(c);
 }
+// blocks, threads and shared memory of the x passes over `lines` lines of length n
+template <typename C, int N> struct XLaunch {
+  int blocks, threads;
+  size_t smem;
+  XLaunch(long lines, int n)
+      : blocks(nblk(lines, N > 0 ? LXD : LX)),
+        threads(N > 0 ? direct_threads(N > 0 ? N : 36, LXD) : NTHR),
+        smem(N > 0 ? (size_t)LXD * (N + 1) * sizeof(C) : x_smem<C>(n)) {}
+};
 template <typename C> static void x_fwd(amdk_ctx *c, int sphere, int T, const XBufs &b = XBufs{}) {
   const Geom &g = c->geom;
   long lines = (long)T * g.nray[sphere];
@@ -392,34 +427,38 @@ template <typename C> static void x_fwd(amdk_ctx *c, int sphere, int T, const XB
   with_n(g.n1, [&](auto NC) {
     constexpr int N = decltype(NC)::value;
     smem_opt_in<k_x_fwd<C, N>>();
-    k_x_fwd<C, N><<<nblk(lines, LX), NTHR, x_smem<C>(g.n1), c->st>>>(sphere, T, g, plan<C>(c, 0),
-                                                                     (C *)rays_of(c, sphere, b));
+    const XLaunch<C, N> L(lines, g.n1);
+    k_x_fwd<C, N><<<L.blocks, L.threads, L.smem, c->st>>>(sphere, T, g, plan<C>(c, 0), fft_tw<C, N>(),
+                                                         (C *)rays_of(c, sphere, b));
   });
   prof_end(c);
 }
 
-// T fields on the density sphere (SRC: see k_x_bwd_field) -> real or complex
-// grids (FP64 in and out; C is the precision of the transform itself)
+// T fields on the density sphere (SRC: see k_x_bwd_field) -> complex grids, or
+// the real parts into real grids where rgrid is given (FP64 in and out; C is
+// the precision of the transform itself)
 template <typename C = double2, int SRC = FS_REAL>
 static int field_to_grid(amdk_ctx *c, int T, const double2 *f, double2 *cgrid,
-                         const XBufs &b = XBufs{}) {
+                         double *rgrid = nullptr, const XBufs &b = XBufs{}) {
   const Geom &g = c->geom;
   long lines = (long)T * g.nray[1];
   ++c->nlaunch;
   with_n(g.n1, [&](auto NC) {
     constexpr int N = decltype(NC)::value;
     smem_opt_in<k_x_bwd_field<C, N, SRC>>();
-    k_x_bwd_field<C, N, SRC><<<nblk(lines, LX), NTHR, x_smem<C>(g.n1), c->st>>>(
-        f, c->d_gvec, c->hs.tpiba, g.ngrho, 1, T, g, plan<C>(c, 0), (C *)rays_of(c, 1, b));
+    const XLaunch<C, N> L(lines, g.n1);
+    k_x_bwd_field<C, N, SRC><<<L.blocks, L.threads, L.smem, c->st>>>(f, c->d_gvec, c->hs.tpiba, g.ngrho, 1, T, g,
+                                                                   plan<C>(c, 0), fft_tw<C, N>(), (C *)rays_of(c, 1, b));
   });
   y_pass<C>(c, 1, +1, T, b);
-  z_pass<C, Z_TO_GRID>(c, 1, T, cgrid, nullptr, 0, b);
+  if (rgrid) z_pass<C, Z_TO_REAL>(c, 1, T, nullptr, rgrid, 0, b);
+  else z_pass<C, Z_TO_GRID>(c, 1, T, cgrid, nullptr, 0, b);
   return 0;
 }
 // T complex grids (or one real grid) -> forward transform left in the ray buffer
 template <typename C = double2>
 static int grid_to_rays(amdk_ctx *c, int T, const double2 *cgrid, const double *rgrid, const XBufs &b = XBufs{}) {
-  if (rgrid) z_pass<C, Z_FROM_GRID_REAL>(c, 1, 1, nullptr, rgrid, 0, b);
+  if (rgrid) z_pass<C, Z_FROM_GRID_REAL>(c, 1, 1, nullptr, (double *)rgrid, 0, b);
   else z_pass<C, Z_FROM_GRID_CPLX>(c, 1, T, (double2 *)cgrid, nullptr, 0, b);
   y_pass<C>(c, 1, -1, T, b);
   x_fwd<C>(c, 1, T, b);
@@ -429,23 +468,6 @@ static int grid_to_rays(amdk_ctx *c, int T, const double2 *cgrid, const double *
 // ------------------------------------------------------------------ pencil path
 // elements of the ray buffer per pair on the pencil path
 static long pencil_stride(const amdk_ctx *c) { return (long)c->pg.nray * c->geom.n1; }
-// the twiddle tables of a length, a kernel parameter
-template <typename C, int N> static const PencilTw<C, N> &pencil_tw() {
-  static const PencilTw<C, N> t = []() {
-    PencilTw<C, N> x;
-    constexpr int N1 = fft_n1(N), N2 = N / N1;
-    const double tp = 8.0 * std::atan(1.0);
-    for (int i = 0; i < N; ++i)
-      for (int h = 0; h < 2; ++h) {
-        const int d = h ? N2 : N1, e = (i / d) * (i % d) % N;
-        const double a = -tp * (double)e / (double)N;
-        x.t[h * N + i].x = (decltype(x.t[0].x))std::cos(a);
-        x.t[h * N + i].y = (decltype(x.t[0].x))std::sin(a);
-      }
-    return x;
-  }();
-  return t;
-}
 // resident blocks per SM of a pencil kernel
 template <auto K> static int pencil_resident(int nt, size_t smem) {
   static const int nb = [&]() {
@@ -496,7 +518,7 @@ static void launch_pencil_vpsi(int nsm, const PencilGeom &pg, C *rb, const void 
   typedef VpsiShape<C, N> Sh;
   constexpr auto K = k_pencil_vpsi<C, N, SEG, LSD>;
   const int units = pg.n1 * T, grid = std::min(units, nsm * pencil_resident<K>(Sh::NT, Sh::smem));
-  K<<<grid, Sh::NT, Sh::smem, st>>>(pg, pencil_tw<C, N>(), rb, (const Rl *)vt, units, (C *)scratch, (const Rl *)vt2, gp0,
+  K<<<grid, Sh::NT, Sh::smem, st>>>(pg, fft_tw<C, N>(), rb, (const Rl *)vt, units, (C *)scratch, (const Rl *)vt2, gp0,
                                     psplit, pstraddle);
 }
 // bytes of the ray shares between column groups of launch_pencil_vpsi (0: not used)
@@ -542,7 +564,7 @@ static void launch_pencil_density(int nsm, const PencilGeom &pg, const C *rb, in
   typedef DensShape<C, N> Sh;
   constexpr auto K = k_pencil_density<C, N, SEG>;
   const int nblk = (int)std::min<long>((long)pg.n1 * Sh::GA * T, (long)nsm * pencil_resident<K>(Sh::NT, Sh::smem));
-  K<<<nblk, Sh::NT, Sh::smem, st>>>(pg, pencil_tw<C, N>(), rb, T, wa, wb, part);
+  K<<<nblk, Sh::NT, Sh::smem, st>>>(pg, fft_tw<C, N>(), rb, T, wa, wb, part);
   constexpr int n1f = fft_n1(N);
   k_rho_reduce_p<<<dim3((N + 31) / 32, (pg.n1 + 31) / 32, N), dim3(32, 8), 0, st>>>(N, pg.n1, n1f, N / n1f, Sh::Z1,
                                                                                   Sh::GA, part, rho, add, T, nblk);
@@ -642,22 +664,18 @@ static int do_density(amdk_ctx *c) {
   return density_t<double2>(c);
 }
 
-// V(r) (real part of a complex grid) into vpot and, on the pencil path, its
-// permuted copy vt for the V(r)psi kernel
-static int store_potential(amdk_ctx *c, const double2 *grid, double *vpot, void *vt) {
+// V(r) from V(G) into vpot (the real part of the backward transform,
+// xc.f90:299-301) and, on the pencil path, its permuted copy vt for the V(r)psi
+// kernel
+template <typename C> static int store_potential(amdk_ctx *c, const double2 *vg, double *vpot, void *vt) {
   const Geom &g = c->geom;
-  const long npt = (long)g.n1 * g.n2 * g.n3;
-  if (!c->pencil_vpsi) {
-    CK(cudaMemcpy2DAsync(vpot, sizeof(double), grid, sizeof(double2), sizeof(double), npt, cudaMemcpyDeviceToDevice,
-                         c->st));
-  } else {
-    dim3 gt((g.n1 + 31) / 32, (g.n1 + 31) / 32, g.n1);
-    const int n1f = fft_n1(g.n1), n2f = g.n1 / n1f;
+  typedef decltype(C().x) Rl;
+  RC(field_to_grid<C>(c, 1, vg, nullptr, vpot));
+  if (c->pencil_vpsi) {
+    const int n1f = fft_n1(g.n1);
     ++c->nlaunch;
-    if (c->precision == AMDK_MIXED)
-      k_v_store<float><<<gt, dim3(32, 8), 0, c->st>>>(g.n1, n1f, n2f, grid, vpot, (float *)vt);
-    else
-      k_v_store<double><<<gt, dim3(32, 8), 0, c->st>>>(g.n1, n1f, n2f, grid, vpot, (double *)vt);
+    k_v_permute<Rl><<<dim3((g.n1 + 31) / 32, (g.n1 + 31) / 32, g.n1), dim3(32, 8), 0, c->st>>>(g.n1, g.n1, n1f,
+                                                                                            g.n1 / n1f, vpot, (Rl *)vt);
   }
   return 0;
 }
@@ -689,8 +707,7 @@ template <typename C> static int potential_lsd_t(amdk_ctx *c) {
                                                        scale, c->d_gvec, h.tpiba, c->d_vg, vx[sp]);
   }
   for (int sp = 0; sp < 2; ++sp) {
-    RC(field_to_grid<C>(c, 1, vx[sp], c->d_cgrid));
-    RC(store_potential(c, c->d_cgrid, sp ? c->d_vpot2 : c->d_vpot, sp ? c->d_vt2 : c->d_vt));
+    RC(store_potential<C>(c, vx[sp], sp ? c->d_vpot2 : c->d_vpot, sp ? c->d_vt2 : c->d_vt));
   }
   CK(cudaGetLastError());
   return 0;
@@ -732,10 +749,8 @@ template <typename C> static int potential_t(amdk_ctx *c, bool gather = false) {
   ++c->nlaunch;
   k_xc_combine<C><<<nblk(h.ngrho), NTHR, 0, c->st>>>(h.ngrho, gga, c->d_posp, c->d_posm, (C *)c->d_rbf, rstride(c, 1),
                                                      scale, c->d_gvec, h.tpiba, c->d_vg, c->d_vxg);
-  RC(field_to_grid<C>(c, 1, c->d_vxg, c->d_cgrid));
-  // V(r) = Re of the backward transform (xc.f90:299-301), and V in the
-  // x-plane-major layout the pencil kernel reads
-  RC(store_potential(c, c->d_cgrid, c->d_vpot, c->d_vt));
+  // V(r), and V in the x-plane-major layout the pencil kernel reads
+  RC(store_potential<C>(c, c->d_vxg, c->d_vpot, c->d_vt));
   CK(cudaGetLastError());
   return 0;
 }
@@ -1479,6 +1494,8 @@ static int build_device(amdk_ctx *c) {
     g.nz[S] = (int)zl.size();
     RC(c->up(&c->d_zlist[S], zl));
     RC(c->up(&c->d_rayidx[S], ri));
+    RC(c->up(&c->d_zinv[S], zi_of));
+    g.zinv[S] = c->d_zinv[S];
     g.zlist[S] = c->d_zlist[S];
     g.rayidx[S] = c->d_rayidx[S];
   }
@@ -2877,7 +2894,7 @@ int amdk_fft_sphere_noalloc(amdk_ctx *c, int sign, double *coef, double *grid) {
   const long npt = (long)h.nr[0] * h.nr[1] * h.nr[2];
   if (sign == -1) {
     // coef (+G half) -> complex grid; the -G values are conj(coef)
-    RC(field_to_grid<double2>(c, 1, (const double2 *)coef, (double2 *)grid, b));
+    RC(field_to_grid<double2>(c, 1, (const double2 *)coef, (double2 *)grid, nullptr, b));
   } else {
     // complex grid -> coef = F(+G)/N
     RC(grid_to_rays<double2>(c, 1, (const double2 *)grid, nullptr, b));

@@ -9,14 +9,16 @@
 //            R[t][ray][kx]
 //   Y pass : the z planes that contain rays (the slab), layout S[t][zi][ky][kx]
 //   Z pass : every (kx,ky) column of the full grid
-// Each pass loads a tile of lines into shared memory (x-fastest global tiles,
-// coalesced), transforms it (the two-level register FFT for the specialised
-// lengths, a shared-memory Stockham mixed-radix (4,2,3,5) FFT otherwise) and
-// stores the tile.  The Z pass carries the fused consumers: |psi|^2 density
-// accumulation, and V(r)*psi between the backward and forward z transforms
-// (the full grid is never written for H|psi>).  The band-pair transforms of
-// cubic grids take the pencil path of pencil.cuh instead; these kernels
-// serve the density-sphere fields and the other grids.
+// For the specialised lengths a thread takes the elements of its
+// sub-transforms straight from global memory (x-fastest, coalesced) and stores
+// them from registers, with one exchange through shared memory between the
+// two phases; run-time lengths load a tile of lines into shared memory and
+// transform it with a Stockham mixed-radix (4,2,3,5) FFT.  The Z pass of band
+// pairs carries the fused consumers: |psi|^2 density accumulation, and
+// V(r)*psi between the backward and forward z transforms (the full grid is
+// never written for H|psi>).  The band-pair transforms of cubic grids take the
+// pencil path of pencil.cuh instead; these kernels serve the density-sphere
+// fields and the other grids.
 //
 // Index convention: grid index k = (Miller index) mod N, x fastest.  The
 // backward transform is sum_G c(G) exp(+iG.r) (FFTW_BACKWARD, unscaled); the
@@ -390,6 +392,45 @@ __device__ __forceinline__ void twiddle_tab(C (&v)[R], int j, const C *tw) {
   }
 }
 
+// The twiddle tables of a specialised length as a kernel parameter (read from
+// the constant bank): t[j2*N1 + k1] = W_N^(j2 k1), t[N + k1*N2 + k2] =
+// W_N^(k1 k2).  N = 0 (run-time lengths): unused.
+template <typename C, int N> struct FftTw {
+  C t[N > 0 ? 2 * N : 1];
+};
+// Two-level transform of lines that come from and go to global memory, one
+// line per l: load(k) and store(k, value) move element k of the calling
+// thread's line.  Thread (l, h), h < N2: phase A loads its N1 elements straight
+// into registers and leaves them in s[k*ES + l*EL]; after one barrier phase B
+// (h < N1) stores its N2 outputs from registers.  The field transforms are
+// short launches bound by latency (7% of the copy rate): one shared tile and
+// one barrier, where staging the tile in and out took two tiles and three.
+// 100^3 FP64, per launch: y 18.6 -> 10.8 us, forward x 16.1 -> 11.3, backward x
+// 24 -> 12 (gradients 23), z 17-22 -> 8-13.
+template <typename C, int N, int SG, int ES, int EL, typename Load, typename Store>
+__device__ __forceinline__ void line_fft_direct(C *s, int l, int h, bool on, const C *tw, Load &&load, Store &&store) {
+  constexpr int N1 = fft_n1(N), N2 = N / N1;
+  C *line = s + l * EL;
+  if (on && h < N2) {
+    C v[N1];
+#pragma unroll
+    for (int j1 = 0; j1 < N1; ++j1) v[j1] = load(h + N2 * j1);
+    Dft<C, N1, SG>::run(v);
+    twiddle_tab<C, N, N1, SG, 0>(v, h, tw);
+#pragma unroll
+    for (int k1 = 0; k1 < N1; ++k1) line[(k1 * N2 + h) * ES] = v[k1];
+  }
+  __syncthreads();
+  if (on && h < N1) {
+    C u[N2];
+#pragma unroll
+    for (int j2 = 0; j2 < N2; ++j2) u[j2] = line[(h * N2 + j2) * ES];
+    Dft<C, N2, SG>::run(u);
+#pragma unroll
+    for (int k2 = 0; k2 < N2; ++k2) store(h + N1 * k2, u[k2]);
+  }
+}
+
 // Two-level register FFT of a tile of L lines (element k of line l at
 // a[k*ES + l]), natural order in a, natural order out in b: phase A in place
 // in a (thread (l, j2): DFT_N1 of elements j2 + N2*j1, twiddle, back to
@@ -446,10 +487,14 @@ struct Geom {
   int nz[2];              // slab planes per sphere
   const int *zlist[2];    // [nz] kz of each slab plane
   const int *rayidx[2];   // [nz*n2] ray of (zi, ky) or -1
+  const int *zinv[2];     // [n3] slab plane of kz or -1
 };
 
 constexpr int TX = 16;    // x-extent of a Y/Z tile (16 complex = 256 B in FP64)
 constexpr int LX = 8;     // lines per X-pass block
+constexpr int LXD = 16;   // lines per X-pass block of the density-sphere fields (specialised lengths)
+// threads and shared memory of the direct field kernels of length n
+constexpr int direct_threads(int n, int lines) { return lines * (n / fft_n1(n)); }
 
 // ---------------------------------------------------------------- X pass
 // Backward X pass with the band-pair pack fused (vpsi/eval_density pack,
@@ -501,19 +546,13 @@ enum { FS_REAL = 0, FS_GRAD = 1 };
 template <typename C, int N, int SRC>
 __global__ void __launch_bounds__(256) k_x_bwd_field(const double2 *__restrict__ f, const double *__restrict__ gvec,
                                                      double tpiba, int ngmax,
-                                                     int sphere, int T, Geom g, Plan<C> p, C *__restrict__ rb) {
+                                                     int sphere, int T, Geom g, Plan<C> p,
+                                                     const __grid_constant__ FftTw<C, N> ft, C *__restrict__ rb) {
   extern __shared__ unsigned char smraw[];
   C *sa = reinterpret_cast<C *>(smraw);
   const int n1 = g.n1, R = sphere ? g.nray[1] : g.nray[0];
-  const int es = LX + 1;
-  C *sb = sa + n1 * es;
-  C *tw = sb + n1 * es;
-  load_tw<C, N>(tw, p);
-  const long line0 = (long)blockIdx.x * LX;
   const long nlines = (long)T * R;
-  auto gather = [&](int idx) {
-    const int l = idx / n1, k = idx % n1;
-    const long line = line0 + l;
+  auto gather = [&](long line, int k) {
     C v = czero<C>();
     if (line < nlines) {
       const int t = (int)(line / R), r = (int)(line % R);
@@ -539,131 +578,168 @@ __global__ void __launch_bounds__(256) k_x_bwd_field(const double2 *__restrict__
     return v;
   };
   if constexpr (N > 0) {
-    // all of a thread's gathers in flight at once (256 threads per block)
-    constexpr int CNT = (LX * N + 255) / 256;
-    C v[CNT];
-#pragma unroll
-    for (int i = 0; i < CNT; ++i) {
-      const int idx = threadIdx.x + 256 * i;
-      v[i] = idx < LX * N ? gather(idx) : czero<C>();
-    }
-#pragma unroll
-    for (int i = 0; i < CNT; ++i) {
-      const int idx = threadIdx.x + 256 * i;
-      if (idx < LX * N) sa[(idx % N) * es + idx / N] = v[i];
-    }
+    constexpr int N2 = N / fft_n1(N);
+    const int l = threadIdx.x / N2, h = threadIdx.x - l * N2;
+    const long line = (long)blockIdx.x * LXD + l;
+    C *o = rb + line * N;
+    line_fft_direct<C, N, 1, 1, N + 1>(
+        sa, l, h, line < nlines, ft.t, [&](int k) { return gather(line, k); }, [&](int k, const C &v) { o[k] = v; });
   } else {
-    for (int idx = threadIdx.x; idx < LX * n1; idx += blockDim.x) sa[(idx % n1) * es + idx / n1] = gather(idx);
-  }
-  __syncthreads();
-  C *res = fft_tile<C, N, LX, LX + 1>(sa, sb, p, tw, +1);
-  for (int idx = threadIdx.x; idx < LX * n1; idx += blockDim.x) {
-    const int l = idx / n1, k = idx % n1;
-    const long line = line0 + l;
-    if (line < nlines) rb[line * n1 + k] = res[k * es + l];
+    const int es = LX + 1;
+    C *sb = sa + n1 * es;
+    const long line0 = (long)blockIdx.x * LX;
+    for (int idx = threadIdx.x; idx < LX * n1; idx += blockDim.x)
+      sa[(idx % n1) * es + idx / n1] = gather(line0 + idx / n1, idx % n1);
+    __syncthreads();
+    C *res = smem_fft(sa, sb, LX, es, p, +1);
+    for (int idx = threadIdx.x; idx < LX * n1; idx += blockDim.x) {
+      const int l = idx / n1, k = idx % n1;
+      const long line = line0 + l;
+      if (line < nlines) rb[line * n1 + k] = res[k * es + l];
+    }
   }
 }
 
 // Forward X pass in place on the ray buffer.
 template <typename C, int N = 0>
-__global__ void __launch_bounds__(256) k_x_fwd(int sphere, int T, Geom g, Plan<C> p, C *__restrict__ rb) {
+__global__ void __launch_bounds__(256) k_x_fwd(int sphere, int T, Geom g, Plan<C> p,
+                                               const __grid_constant__ FftTw<C, N> ft, C *__restrict__ rb) {
   extern __shared__ unsigned char smraw[];
   C *sa = reinterpret_cast<C *>(smraw);
   const int n1 = g.n1, R = sphere ? g.nray[1] : g.nray[0];
-  const int es = LX + 1;
-  C *sb = sa + n1 * es;
-  C *tw = sb + n1 * es;
-  load_tw<C, N>(tw, p);
-  const long line0 = (long)blockIdx.x * LX;
   const long nlines = (long)T * R;
-  for (int idx = threadIdx.x; idx < LX * n1; idx += blockDim.x) {
-    const int l = idx / n1, k = idx % n1;
-    const long line = line0 + l;
-    sa[k * es + l] = (line < nlines) ? rb[line * n1 + k] : czero<C>();
-  }
-  __syncthreads();
-  C *res = fft_tile<C, N, LX, LX + 1>(sa, sb, p, tw, -1);
-  for (int idx = threadIdx.x; idx < LX * n1; idx += blockDim.x) {
-    const int l = idx / n1, k = idx % n1;
-    const long line = line0 + l;
-    if (line < nlines) rb[line * n1 + k] = res[k * es + l];
+  if constexpr (N > 0) {
+    constexpr int N2 = N / fft_n1(N);
+    const int l = threadIdx.x / N2, h = threadIdx.x - l * N2;
+    const long line = (long)blockIdx.x * LXD + l;
+    C *o = rb + line * N;
+    line_fft_direct<C, N, -1, 1, N + 1>(
+        sa, l, h, line < nlines, ft.t, [&](int k) { return o[k]; }, [&](int k, const C &v) { o[k] = v; });
+  } else {
+    const int es = LX + 1;
+    C *sb = sa + n1 * es;
+    const long line0 = (long)blockIdx.x * LX;
+    for (int idx = threadIdx.x; idx < LX * n1; idx += blockDim.x) {
+      const int l = idx / n1, k = idx % n1;
+      const long line = line0 + l;
+      sa[k * es + l] = (line < nlines) ? rb[line * n1 + k] : czero<C>();
+    }
+    __syncthreads();
+    C *res = smem_fft(sa, sb, LX, es, p, -1);
+    for (int idx = threadIdx.x; idx < LX * n1; idx += blockDim.x) {
+      const int l = idx / n1, k = idx % n1;
+      const long line = line0 + l;
+      if (line < nlines) rb[line * n1 + k] = res[k * es + l];
+    }
   }
 }
 
 // ---------------------------------------------------------------- Y pass
-// grid: (ceil(n1/TX), nz[sphere], T).  dir=+1 backward (rays -> slab),
-// dir=-1 forward (slab -> rays).
-template <typename C, int N = 0>
-__global__ void __launch_bounds__(256) k_y(int sphere, int dir, Geom g, Plan<C> p, C *__restrict__ rb, C *__restrict__ sbuf,
-                                           long rstride, long sstride) {
+// grid: (ceil(n1/TX), nz[sphere], T).  DIR=+1 backward (rays -> slab),
+// DIR=-1 forward (slab -> rays).
+template <typename C, int N, int DIR>
+__global__ void __launch_bounds__(256) k_y(int sphere, Geom g, Plan<C> p, const __grid_constant__ FftTw<C, N> ft,
+                                           C *__restrict__ rb, C *__restrict__ sbuf, long rstride, long sstride) {
   extern __shared__ unsigned char smraw[];
   C *sa = reinterpret_cast<C *>(smraw);
-  const int n1 = g.n1, n2 = g.n2, nz = sphere ? g.nz[1] : g.nz[0];
-  C *sb = sa + n2 * TX;
-  C *tw = sb + n2 * TX;
-  load_tw<C, N>(tw, p);
+  const int n1 = g.n1, n2 = g.n2;
   const int kx0 = blockIdx.x * TX, zi = blockIdx.y, t = blockIdx.z;
   const int *ri = (sphere ? g.rayidx[1] : g.rayidx[0]) + (long)zi * n2;
   C *R = rb + (long)t * rstride;
   C *S = sbuf + (long)t * sstride + (long)zi * n2 * n1;
-  auto fetch = [&](int idx) {
-    const int ky = idx / TX, tx = idx % TX, kx = kx0 + tx;
+  auto fetch = [&](int kx, int ky) {
     C v = czero<C>();
-    if (kx < n1) {
-      if (dir > 0) {
-        const int r = ri[ky];
-        if (r >= 0) v = R[(long)r * n1 + kx];
-      } else {
-        v = S[(long)ky * n1 + kx];
-      }
+    if (DIR > 0) {
+      const int r = ri[ky];
+      if (r >= 0) v = R[(long)r * n1 + kx];
+    } else {
+      v = S[(long)ky * n1 + kx];
     }
     return v;
   };
-  if constexpr (N > 0) {
-    // all of a thread's loads in flight at once (256 threads per block)
-    constexpr int CNT = (TX * N + 255) / 256;
-    C v[CNT];
-#pragma unroll
-    for (int i = 0; i < CNT; ++i) {
-      const int idx = threadIdx.x + 256 * i;
-      v[i] = idx < TX * N ? fetch(idx) : czero<C>();
-    }
-#pragma unroll
-    for (int i = 0; i < CNT; ++i) {
-      const int idx = threadIdx.x + 256 * i;
-      if (idx < TX * N) sa[idx] = v[i];
-    }
-  } else {
-    for (int idx = threadIdx.x; idx < TX * n2; idx += blockDim.x) sa[idx] = fetch(idx);
-  }
-  __syncthreads();
-  C *res = fft_tile<C, N, TX, TX>(sa, sb, p, tw, dir);
-  for (int idx = threadIdx.x; idx < TX * n2; idx += blockDim.x) {
-    const int ky = idx / TX, tx = idx % TX, kx = kx0 + tx;
-    if (kx >= n1) continue;
-    if (dir > 0) {
-      S[(long)ky * n1 + kx] = res[ky * TX + tx];
+  auto put = [&](int kx, int ky, const C &v) {
+    if (DIR > 0) {
+      S[(long)ky * n1 + kx] = v;
     } else {
       const int r = ri[ky];
-      if (r >= 0) R[(long)r * n1 + kx] = res[ky * TX + tx];
+      if (r >= 0) R[(long)r * n1 + kx] = v;
+    }
+  };
+  if constexpr (N > 0) {
+    const int l = threadIdx.x % TX, h = threadIdx.x / TX, kx = kx0 + l;
+    line_fft_direct<C, N, DIR, TX, 1>(
+        sa, l, h, kx < n1, ft.t, [&](int k) { return fetch(kx, k); }, [&](int k, const C &v) { put(kx, k, v); });
+  } else {
+    C *sb = sa + n2 * TX;
+    for (int idx = threadIdx.x; idx < TX * n2; idx += blockDim.x) {
+      const int kx = kx0 + idx % TX;
+      sa[idx] = kx < n1 ? fetch(kx, idx / TX) : czero<C>();
+    }
+    __syncthreads();
+    C *res = smem_fft(sa, sb, TX, TX, p, DIR);
+    for (int idx = threadIdx.x; idx < TX * n2; idx += blockDim.x) {
+      const int kx = kx0 + idx % TX;
+      if (kx < n1) put(kx, idx / TX, res[idx]);
     }
   }
-  (void)nz;
 }
 
 // ---------------------------------------------------------------- Z pass
-enum { Z_TO_GRID = 0, Z_FROM_GRID_REAL = 1, Z_FROM_GRID_CPLX = 2, Z_VPSI = 3, Z_DENSITY = 4 };
+enum { Z_TO_GRID = 0, Z_FROM_GRID_REAL = 1, Z_FROM_GRID_CPLX = 2, Z_VPSI = 3, Z_DENSITY = 4, Z_TO_REAL = 5 };
 
 // grid: (ceil(n1/TX), n2, T) for TO_GRID/FROM_GRID/VPSI; (ceil(n1/TX), n2, 1)
 // for DENSITY, which loops over the T transforms of the batch.
 //   TO_GRID          slab -> complex grid (double2)                    backward
+//   TO_REAL          slab -> real part, a real grid (double)           backward
 //   FROM_GRID_REAL   real grid (double) -> slab                        forward
 //   FROM_GRID_CPLX   complex grid (double2) -> slab                    forward
 //   VPSI             slab -> (bwd) * V(r) -> (fwd) -> slab  (vpsi, wfn_initialize.f90:311-340)
 //   DENSITY          slab -> (bwd) -> rho += f_a/Omega Re^2 + f_b/Omega Im^2 (density.f90:49-86)
+// The field modes of specialised lengths move their lines directly between
+// global memory and registers (k_z_field below); k_z has the pair modes and
+// the run-time lengths.
+template <typename C, int MODE, int N>
+__global__ void __launch_bounds__(256) k_z_field(int sphere, Geom g, const __grid_constant__ FftTw<C, N> ft,
+                                                 C *__restrict__ sbuf, long sstride, double2 *__restrict__ cgrid,
+                                                 double *__restrict__ rgrid, long gstride) {
+  typedef decltype(C().x) R;
+  extern __shared__ unsigned char smraw[];
+  const int n1 = g.n1, n2 = g.n2;
+  const int l = threadIdx.x % TX, h = threadIdx.x / TX, kx = blockIdx.x * TX + l, ky = blockIdx.y;
+  const int *zinv = sphere ? g.zinv[1] : g.zinv[0];
+  const long plane = (long)n2 * n1, at = (long)ky * n1 + kx;
+  C *S = sbuf + (long)blockIdx.z * sstride + at;
+  double2 *G = cgrid + (long)blockIdx.z * gstride + at;
+  double *Q = rgrid + (long)blockIdx.z * gstride + at;
+  constexpr bool BWD = MODE == Z_TO_GRID || MODE == Z_TO_REAL;
+  line_fft_direct<C, N, BWD ? 1 : -1, TX, 1>(
+      reinterpret_cast<C *>(smraw), l, h, kx < n1, ft.t,
+      [&](int kz) {
+        C v = czero<C>();
+        if (BWD) {
+          const int zi = zinv[kz];
+          if (zi >= 0) v = S[zi * plane];
+        } else if (MODE == Z_FROM_GRID_REAL) {
+          v.x = (R)Q[kz * plane];
+        } else {
+          const double2 c = G[kz * plane];
+          v = mk((R)c.x, (R)c.y);
+        }
+        return v;
+      },
+      [&](int kz, const C &v) {
+        if (MODE == Z_TO_GRID) G[kz * plane] = make_double2((double)v.x, (double)v.y);
+        else if (MODE == Z_TO_REAL) Q[kz * plane] = (double)v.x;
+        else {
+          const int zi = zinv[kz];
+          if (zi >= 0) S[zi * plane] = v;
+        }
+      });
+}
+
 template <typename C, int MODE, int N = 0>
 __global__ void __launch_bounds__(256) k_z(int sphere, int T, Geom g, Plan<C> p, C *__restrict__ sbuf, long sstride,
-                                           double2 *__restrict__ cgrid, const double *__restrict__ rgrid, long gstride,
+                                           double2 *__restrict__ cgrid, double *__restrict__ rgrid, long gstride,
                                            const double *__restrict__ vpot, double *__restrict__ rho,
                                            const double *__restrict__ wa, const double *__restrict__ wb) {
   typedef decltype(C().x) R;
@@ -683,7 +759,7 @@ __global__ void __launch_bounds__(256) k_z(int sphere, int T, Geom g, Plan<C> p,
   const int te = (MODE == Z_DENSITY) ? T : blockIdx.z + 1;
   for (int t = tb; t < te; ++t) {
     C *S = sbuf + (long)t * sstride;
-    if (MODE == Z_TO_GRID || MODE == Z_VPSI || MODE == Z_DENSITY) {
+    if (MODE == Z_TO_GRID || MODE == Z_TO_REAL || MODE == Z_VPSI || MODE == Z_DENSITY) {
       if constexpr (N > 0) {
         // the slab loads are issued before the clearing barrier (256 threads per block)
         constexpr int CNT = (TX * N + 255) / 256;
@@ -724,6 +800,13 @@ __global__ void __launch_bounds__(256) k_z(int sphere, int T, Geom g, Plan<C> p,
             C v = res[idx];
             G[(long)kz * plane + (long)ky * n1 + kx] = make_double2((double)v.x, (double)v.y);
           }
+        }
+        __syncthreads();
+      } else if (MODE == Z_TO_REAL) {
+        double *G = rgrid + (long)t * gstride;
+        for (int idx = threadIdx.x; idx < TX * n3; idx += blockDim.x) {
+          const int kz = idx / TX, tx = idx % TX, kx = kx0 + tx;
+          if (kx < n1) G[(long)kz * plane + (long)ky * n1 + kx] = (double)res[idx].x;
         }
         __syncthreads();
       } else if (MODE == Z_DENSITY) {

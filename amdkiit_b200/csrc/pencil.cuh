@@ -194,12 +194,6 @@ template <int N, int M1 = fft_n1(N)> struct Sphere {
   }
 };
 
-// The twiddle tables of a pencil kernel as a kernel parameter (the constant
-// bank): t[j2*N1 + k1] = W_N^(j2 k1), t[N + k1*N2 + k2] = W_N^(k1 k2)
-template <typename C, int N> struct PencilTw {
-  C t[2 * N];
-};
-
 // Rays of a slab plane.  SEG = false (one GPU): the rays of a ky are those of
 // kz = lo .. hi (signed), consecutive in the buffer; SEG = true (the segments
 // of a slab decomposition): looked up per (ky, zi).  Each thread (row zi, j2)
@@ -434,7 +428,7 @@ template <typename C, int N> struct PencilSmem {
 // (wfn_initialize.f90:313-326).
 template <typename C, int N, bool SEG, bool LSD>
 __global__ void __launch_bounds__(VpsiShape<C, N>::NT, VpsiShape<C, N>::MINB)
-    k_pencil_vpsi(const PencilGeom pg, const __grid_constant__ PencilTw<C, N> p, C *__restrict__ rt,
+    k_pencil_vpsi(const PencilGeom pg, const __grid_constant__ FftTw<C, N> p, C *__restrict__ rt,
                   const decltype(C().x) *__restrict__ vp, int units, C *__restrict__ scratch,
                   const decltype(C().x) *__restrict__ vp2, int gp0, int psplit, int pstraddle) {
   typedef decltype(C().x) Rl;
@@ -605,7 +599,7 @@ __host__ __device__ __forceinline__ int bal_slots(int kx, int T, long U, int nbl
 }
 template <typename C, int N, bool SEG>
 __global__ void __launch_bounds__(DensShape<C, N>::NT, DensShape<C, N>::MINB)
-    k_pencil_density(const PencilGeom pg, const __grid_constant__ PencilTw<C, N> p, const C *__restrict__ rt, int T,
+    k_pencil_density(const PencilGeom pg, const __grid_constant__ FftTw<C, N> p, const C *__restrict__ rt, int T,
                      const double *__restrict__ wa, const double *__restrict__ wb, double *__restrict__ rho_part) {
   typedef decltype(C().x) Rl;
   typedef DensShape<C, N> Sh;
@@ -774,31 +768,6 @@ __global__ void k_v_permute(int n, int nx, int n1f, int n2f, const double *__res
   for (int j = threadIdx.y; j < 32; j += blockDim.y) {
     const int kx = kx0 + j, q = q0 + threadIdx.x;
     if (kx < nx && q < n) vp[((long)kx * n + kp) * n + q] = (Rl)tile[threadIdx.x][j];
-  }
-}
-
-// The same from the real part of a complex grid, which is stored in v as well
-template <typename Rl>
-__global__ void k_v_store(int n, int n1f, int n2f, const double2 *__restrict__ grid, double *__restrict__ v,
-                          Rl *__restrict__ vp) {
-  __shared__ double tile[32][33];
-  const int kp = blockIdx.z;
-  const int kz = perm_index(kp, n1f, n2f);
-  const int kx0 = blockIdx.x * 32, q0 = blockIdx.y * 32;
-  for (int j = threadIdx.y; j < 32; j += blockDim.y) {
-    const int q = q0 + j, kx = kx0 + threadIdx.x;
-    double x = 0.0;
-    if (kx < n && q < n) {
-      const long o = ((long)kz * n + perm_index(q, n1f, n2f)) * n + kx;
-      x = grid[o].x;
-      v[o] = x;
-    }
-    tile[j][threadIdx.x] = x;
-  }
-  __syncthreads();
-  for (int j = threadIdx.y; j < 32; j += blockDim.y) {
-    const int kx = kx0 + j, q = q0 + threadIdx.x;
-    if (kx < n && q < n) vp[((long)kx * n + kp) * n + q] = (Rl)tile[threadIdx.x][j];
   }
 }
 
