@@ -133,7 +133,7 @@ struct amdk_ctx {
   unsigned *d_ticket = nullptr;  // tickets of the self-finishing reductions (TK_*)
   // pencil path (cubic grids with a specialised length): tables and buffers
   bool pencil_vpsi = false, pencil_density = false;
-  double *h_pin = nullptr;  // pinned: scalar slots [S_NSCAL], GEMAX, CG step
+  double *h_pin = nullptr;  // pinned: scalar slots [S_NSCAL], CG step
   // CUDA graphs of the CG iteration's two segments (before and after the
   // GEMAX read), keyed by segment, precision/forces flag, which buffer holds
   // C0, and profiling
@@ -1190,10 +1190,13 @@ static int do_gradient(amdk_ctx *c) {
   return 0;
 }
 
-// the CG step number, from pinned host memory (h_pin[S_NSCAL + 1], set before
-// the launch, so that a captured graph of this copy takes the current one)
+// The CG step number of an iteration, from pinned host memory (h_pin[S_NSCAL],
+// set before the launch, so that a captured graph of this copy takes the
+// current one).  Only the iteration entries use the slot, and each waits for
+// segment A, this copy in it, before the update: no copy that an update still
+// needs is under way when the slot is set again.
 static int copy_istep(amdk_ctx *c) {
-  CK(cudaMemcpyAsync(c->d_scal + S_ISTEP, c->h_pin + S_NSCAL + 1, sizeof(double), cudaMemcpyHostToDevice, c->st));
+  CK(cudaMemcpyAsync(c->d_scal + S_ISTEP, c->h_pin + S_NSCAL, sizeof(double), cudaMemcpyHostToDevice, c->st));
   return 0;
 }
 // PCG with the step number in S_ISTEP and the gradient norm S_GG of the
@@ -2510,9 +2513,8 @@ int amdk_gradient(amdk_ctx *c, double *gemax) {
 int amdk_pcg(amdk_ctx *c, int istep) {
   if (!c || istep < 1) return AMDK_ERR_BADARG;
   cudaSetDevice(c->device);
-  CK(cudaStreamSynchronize(c->st));  // an earlier copy of the step number may still read the pinned slot
-  c->h_pin[S_NSCAL + 1] = (double)istep;
-  RC(copy_istep(c));
+  ++c->nlaunch;
+  k_set_scalar<<<1, 1, 0, c->st>>>(c->d_scal + S_ISTEP, (double)istep);  // by value: this entry returns without a wait
   gmax_precon(c);  // the caller may have changed C2 since the gradient
   return do_pcg(c);
 }
@@ -2524,7 +2526,7 @@ int amdk_scf_iteration(amdk_ctx *c, int istep, double gcut, amdk_energies *e, do
   // graphs from the second iteration on, once this precision has run eagerly
   // (first-call setup of kernels and cuBLAS stays out of the capture)
   const bool graph = c->use_graphs && istep > 1 && c->warm[q];
-  c->h_pin[S_NSCAL + 1] = (double)istep;  // copied by segment A; nothing of this context is in flight
+  c->h_pin[S_NSCAL] = (double)istep;  // copied by segment A (copy_istep)
   cudaEventRecord(c->ev0, c->st);
   auto seg_a = [&]() -> int { return seg_a_body(c); };
   if (graph) RC(run_segment(c, seg_a_key(c), seg_a));
@@ -2615,7 +2617,7 @@ int amdk_ensemble_iteration(amdk_ensemble *E, const int *istep, double gcut, amd
     for (int i = 0; i < n; ++i) {
       amdk_ctx *c = E->m[i];
       keys[i] = b ? seg_b_key(c) : seg_a_key(c);
-      if (!b) c->h_pin[S_NSCAL + 1] = (double)istep[i];
+      if (!b) c->h_pin[S_NSCAL] = (double)istep[i];
       sgs[i] = b ? ensure_segment(c, keys[i], [&]() -> int { return seg_b_body(c); })
                  : ensure_segment(c, keys[i], [&]() -> int { return seg_a_body(c); });
       if (!sgs[i]) {

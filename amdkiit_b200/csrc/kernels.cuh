@@ -754,6 +754,7 @@ __global__ void k_gmax_precon(int ngpw, int nocc, const double *vpp, const doubl
   const double vals[2] = {sqrt(m), s};  // sqrt is monotonic: the max of the roots is the root of the max
   reduce_and_finish<2, 1u>(vals, part, out, ticket);
 }
+__global__ void k_set_scalar(double *dst, double v) { *dst = v; }
 // PCG direction and step (cg.f90:109-143) with cp = f_i^-1 K(G) C2 (PRECON,
 // cg.f90:281-311); gamma = forget * ggnorm(new) / ggnorm(previous)
 // The last block to have read the scalars makes the norm the previous one.

@@ -1,0 +1,56 @@
+"""Entries that return before their work has run, followed at once by one that
+sets host or device state of its own: the results are those of the same calls
+with a wait between them, bit for bit."""
+import numpy as np
+import pytest
+
+from amdkiit_b200 import configs
+from amdkiit_b200.engine import FP64, MIXED, Engine
+from amdkiit_b200.inputs import XC_PBE
+from tests.helpers import start_coefficients
+
+pytestmark = pytest.mark.gpu
+
+
+def _engine(system, prec):
+    e = Engine(system, prec)
+    g = e.gvectors()
+    e.set_wfn(start_coefficients(g["hg"][: e.ngpw], 2 * np.pi / system.alat, e.nstate))
+    e.ortho()
+    return e
+
+
+def _stages(e):
+    """One CG iteration up to the gradient by its single entries."""
+    e.density()
+    e.potential()
+    e.energy()
+    e.apply_h()
+    e.gradient()
+
+
+@pytest.mark.parametrize("prec", [FP64, MIXED])
+def test_cg_step_followed_by_an_iteration(prec):
+    """amdk_pcg(a) and amdk_scf_iteration(b) straight after it: each update
+    takes its own step number (a = 1 restarts the direction, b = 12 carries it
+    on with another factor), eager and replayed from graphs."""
+    s = configs.small_water(xc=XC_PBE)
+    got = []
+    for wait in (True, False):
+        e = _engine(s, prec)
+        for it in (1, 2):
+            e.scf_iteration(it, 1e-7)
+        for a, b in ((1, 12), (12, 1), (1, 25)):
+            _stages(e)
+            e.pcg(a)
+            if wait:
+                e.get_wfn()
+            e.scf_iteration(b, 1e-7)
+        _stages(e)
+        e.pcg(1)
+        if wait:
+            e.get_wfn()
+        e.pcg(12)  # the direction of the first carried on
+        got.append(e.get_wfn())
+        e.close()
+    assert np.array_equal(got[0], got[1])
