@@ -2631,6 +2631,14 @@ int amdk_ensemble_iteration(amdk_ensemble *E, const int *istep, double gcut, amd
     for (int i = 0; i < n; ++i) account_segment(E->m[i], *sgs[i]);
     return 0;
   };
+  // work that a member's earlier entries left on its stream (an ortho's
+  // rotation, a CG update) comes first
+  for (amdk_ctx *c : E->m)
+    if (cudaStreamQuery(c->st) != cudaSuccess) {
+      cudaGetLastError();  // not ready
+      CK(cudaEventRecord(c->ev0, c->st));
+      CK(cudaStreamWaitEvent(E->st, c->ev0, 0));
+    }
   CK(cudaEventRecord(E->ev0, E->st));
   RC(run_all(false));
   CK(cudaStreamSynchronize(E->st));

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from amdkiit_b200 import configs
-from amdkiit_b200.engine import FP64, MIXED, Engine
+from amdkiit_b200.engine import FP64, MIXED, Engine, Ensemble
 from amdkiit_b200.inputs import XC_PBE
 from tests.helpers import start_coefficients
 
@@ -54,3 +54,30 @@ def test_cg_step_followed_by_an_iteration(prec):
         got.append(e.get_wfn())
         e.close()
     assert np.array_equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("prec", [FP64, MIXED])
+def test_ensemble_after_work_on_the_members_streams(prec):
+    """An ensemble iteration (its own stream) starts after what its members'
+    entries have queued: the CG update and the rotation of an ortho."""
+    systems = [configs.cluster(n, L, 500 + n, ecut=30.0) for n, L in ((3, 13.5), (2, 14.0))]
+    got = []
+    for wait in (True, False):
+        members = [_engine(s, prec) for s in systems]
+        ens = Ensemble(members)
+        for it in (1, 2, 3):
+            ens.iteration([it] * 2, 1e-7)
+        for it in (4, 5):
+            for e in members:
+                _stages(e)
+                e.pcg(it)
+                e.ortho()
+                if wait:
+                    e.get_wfn()
+            ens.iteration([it] * 2, 1e-7)
+        got.append([e.get_wfn() for e in members])
+        ens.close()
+        for e in members:
+            e.close()
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
