@@ -509,6 +509,11 @@ template <typename C> static void xt_fwd(amdk_ctx *c, int T) {
   });
   prof_end(c);
 }
+// most blocks of a V(r)psi launch: one resident wave
+template <typename C, int N, bool SEG, bool LSD> static int vpsi_blocks(int nsm) {
+  typedef VpsiShape<C, N> Sh;
+  return nsm * pencil_resident<k_pencil_vpsi<C, N, SEG, LSD>>(Sh::NT, Sh::smem);
+}
 // V(r)psi on T pairs of nplane x planes (pg's buffer rb), one wave of
 // persistent blocks
 template <typename C, int N, bool SEG, bool LSD>
@@ -516,19 +521,23 @@ static void launch_pencil_vpsi(int nsm, const PencilGeom &pg, C *rb, const void 
                                const void *vt2, int gp0, int psplit, int pstraddle, cudaStream_t st) {
   typedef decltype(C().x) Rl;
   typedef VpsiShape<C, N> Sh;
-  constexpr auto K = k_pencil_vpsi<C, N, SEG, LSD>;
-  const int units = pg.n1 * T, grid = std::min(units, nsm * pencil_resident<K>(Sh::NT, Sh::smem));
-  K<<<grid, Sh::NT, Sh::smem, st>>>(pg, fft_tw<C, N>(), rb, (const Rl *)vt, units, (C *)scratch, (const Rl *)vt2, gp0,
-                                    psplit, pstraddle);
+  const int units = pg.n1 * T, grid = std::min(units, vpsi_blocks<C, N, SEG, LSD>(nsm));
+  k_pencil_vpsi<C, N, SEG, LSD><<<grid, Sh::NT, Sh::smem, st>>>(pg, fft_tw<C, N>(), rb, (const Rl *)vt, units, (C *)scratch,
+                                                                (const Rl *)vt2, gp0, psplit, pstraddle);
 }
-// bytes of the ray shares between column groups of launch_pencil_vpsi (0: not used)
+// bytes of the ray shares between column groups of launch_pencil_vpsi (0: not
+// used): a plane for each block of the widest launch
 template <typename C> static size_t vpsi_scratch_bytes(int n, int nsm) {
   size_t b = 0;
   with_n(n, [&](auto NC) {
     constexpr int N = decltype(NC)::value;
     if constexpr (N > 0) {
       constexpr size_t nz = Sphere<N>::NZ;
-      if (VpsiShape<C, N>::GA > 1) b = (size_t)nsm * VpsiShape<C, N>::MINB * nz * nz * sizeof(C);
+      if constexpr (VpsiShape<C, N>::GA > 1) {
+        const int nb = std::max({vpsi_blocks<C, N, false, false>(nsm), vpsi_blocks<C, N, false, true>(nsm),
+                                 vpsi_blocks<C, N, true, false>(nsm)});
+        b = (size_t)nb * nz * nz * sizeof(C);
+      }
     }
   });
   return b;

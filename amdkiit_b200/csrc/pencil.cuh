@@ -611,7 +611,7 @@ __global__ void __launch_bounds__(DensShape<C, N>::NT, DensShape<C, N>::MINB)
   C *P = sm.P, *S = sm.S;
   sm.load(pg);
   const C *tw = p.t;
-  const int U = pg.n1 * GA * T, nb = gridDim.x, b = blockIdx.x;  // the launch keeps U within an int
+  const int U = pg.n1 * GA * T, nb = gridDim.x, b = blockIdx.x;  // within an int: more units would have more rays than the card holds
   const int u0 = (int)((long)b * U / nb), u1 = (int)((long)(b + 1) * U / nb);
   const int k1t = threadIdx.x / W, qqt = threadIdx.x - k1t * W;
   Rl acc[NS][Z2];
