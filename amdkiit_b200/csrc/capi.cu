@@ -1471,6 +1471,24 @@ static void pencil_rays(int n, const std::vector<int> &ray_ky, const std::vector
   }
 }
 
+// Whether the rays of all band pairs can be held at once (then the density and
+// H|psi> share an x pass and the iteration has its side stream); else batches
+// of 8.  The rays of all pairs take about three times C0 (160^3, 512 bands:
+// 3.2 GB in FP64), so they have to leave the rest of the context its room: the
+// projector arrays, the predictor's history at its longest and 256 MB for the
+// tables and partial sums.
+static bool rays_fit(const amdk_ctx *c, size_t bytes) {
+  const HostSetup &h = c->hs;
+  size_t free_bytes = 0, total = 0;
+  if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  size_t rows = (size_t)amdk_ctx::MAX_PRED * h.nstate;
+  for (int is = 0; is < h.nsp; is++) rows += 4 * (size_t)h.na[is] * h.ngh[is];
+  return bytes + rows * h.ngpw * sizeof(double2) + ((size_t)256 << 20) <= free_bytes;
+}
+
 static int build_device(amdk_ctx *c) {
   HostSetup &h = c->hs;
   Geom &g = c->geom;
@@ -1640,12 +1658,12 @@ static int build_device(amdk_ctx *c) {
   RC(sg_setup(c));
   const int q0 = (c->precision == AMDK_MIXED) ? 1 : 0;
   const bool pencil_all = c->pv_p[q0] && c->pd_p[q0];
-  // pair batch: all pairs at once on the pencil path, else 8
-  if (c->batch <= 0) c->batch = pencil_all ? c->npairs : 8;
-  c->batch = std::max(1, std::min(c->batch, c->npairs));
   std::vector<int> prays, pcols;  // pencil path: its rays (of the reference's numbering) and table
   if (c->pv_p[0] || c->pv_p[1]) pencil_rays(n1, ray_ky, ray_kz, h.ngrays, prays, pcols);
-  size_t rb = (size_t)c->batch * std::max<long>(rstride(c, 0), (long)prays.size() * n1) * sizeof(double2);
+  const size_t pair_bytes = (size_t)std::max<long>(rstride(c, 0), (long)prays.size() * n1) * sizeof(double2);
+  if (c->batch <= 0) c->batch = pencil_all && rays_fit(c, pair_bytes * c->npairs) ? c->npairs : 8;
+  c->batch = std::max(1, std::min(c->batch, c->npairs));
+  size_t rb = c->batch * pair_bytes;
   const size_t rbf = 2 * (size_t)rstride(c, 1) * sizeof(double2);
   size_t sb = 2 * (size_t)sstride(c, 1) * sizeof(double2);
   if (!(c->pv_p[0] && c->pd_p[0] && c->pv_p[1] && c->pd_p[1]))
