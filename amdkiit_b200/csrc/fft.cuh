@@ -46,12 +46,6 @@ template <typename C> __device__ __forceinline__ C cmul(C a, C b) {
   r.y = a.x * b.y + a.y * b.x;
   return r;
 }
-template <typename C> __device__ __forceinline__ C cconjmul(C a, C b) {  // a * conj(b)
-  C r;
-  r.x = a.x * b.x + a.y * b.y;
-  r.y = a.y * b.x - a.x * b.y;
-  return r;
-}
 template <typename C, typename R> __device__ __forceinline__ C cscale(C a, R s) { a.x *= s; a.y *= s; return a; }
 // i*sg*a
 template <typename C> __device__ __forceinline__ C cimul(C a, int sg) {
@@ -363,32 +357,15 @@ template <typename C, int N> __device__ __forceinline__ void load_tw(C *tw, cons
   }
 }
 // v[k] *= W_N^(SG j k), k = 1..R-1, from row j of twiddle table TAB (table 0
-// for R = N1, j = j2; table 1 for R = N2, j = k1).  VEC: the table starts on a
-// 16-byte boundary (the caller guarantees it), so FP32 rows of even length are
-// read two twiddles per load.
-template <typename C, int N, int R, int SG, int TAB, bool VEC = false>
+// for R = N1, j = j2; table 1 for R = N2, j = k1).
+template <typename C, int N, int R, int SG, int TAB>
 __device__ __forceinline__ void twiddle_tab(C (&v)[R], int j, const C *tw) {
   const C *row = tw + TAB * N + j * R;
-  if constexpr (VEC && sizeof(C) == 8 && R % 2 == 0 && N % 2 == 0) {
-    const float4 *r4 = reinterpret_cast<const float4 *>(row);
 #pragma unroll
-    for (int k2 = 0; k2 < R / 2; ++k2) {
-      const float4 q = r4[k2];
-      C wa, wb;
-      wa.x = q.x;
-      wa.y = SG > 0 ? -q.y : q.y;
-      wb.x = q.z;
-      wb.y = SG > 0 ? -q.w : q.w;
-      if (k2 > 0) v[2 * k2] = cmul(v[2 * k2], wa);
-      v[2 * k2 + 1] = cmul(v[2 * k2 + 1], wb);
-    }
-  } else {
-#pragma unroll
-    for (int k = 1; k < R; ++k) {
-      C w = row[k];
-      if (SG > 0) w.y = -w.y;
-      v[k] = cmul(v[k], w);
-    }
+  for (int k = 1; k < R; ++k) {
+    C w = row[k];
+    if (SG > 0) w.y = -w.y;
+    v[k] = cmul(v[k], w);
   }
 }
 
@@ -742,6 +719,7 @@ __global__ void __launch_bounds__(256) k_z(int sphere, int T, Geom g, Plan<C> p,
                                            double2 *__restrict__ cgrid, double *__restrict__ rgrid, long gstride,
                                            const double *__restrict__ vpot, double *__restrict__ rho,
                                            const double *__restrict__ wa, const double *__restrict__ wb) {
+  static_assert(N == 0 || MODE == Z_VPSI || MODE == Z_DENSITY, "k_z_field has the other modes of a known length");
   typedef decltype(C().x) R;
   extern __shared__ unsigned char smraw[];
   C *sa = reinterpret_cast<C *>(smraw);
@@ -844,22 +822,7 @@ __global__ void __launch_bounds__(256) k_z(int sphere, int T, Geom g, Plan<C> p,
         }
         return v;
       };
-      if constexpr (N > 0) {
-        constexpr int CNT = (TX * N + 255) / 256;
-        C v[CNT];
-#pragma unroll
-        for (int i = 0; i < CNT; ++i) {
-          const int idx = threadIdx.x + 256 * i;
-          v[i] = idx < TX * N ? fetch(idx) : czero<C>();
-        }
-#pragma unroll
-        for (int i = 0; i < CNT; ++i) {
-          const int idx = threadIdx.x + 256 * i;
-          if (idx < TX * N) sa[idx] = v[i];
-        }
-      } else {
-        for (int idx = threadIdx.x; idx < TX * n3; idx += blockDim.x) sa[idx] = fetch(idx);
-      }
+      for (int idx = threadIdx.x; idx < TX * n3; idx += blockDim.x) sa[idx] = fetch(idx);
       __syncthreads();
       C *res = fft_tile<C, N, TX, TX>(sa, sb, p, tw, -1);
       for (int idx = threadIdx.x; idx < TX * nz; idx += blockDim.x) {

@@ -41,16 +41,6 @@ __device__ double block_max(double v, double *sh) {
     for (int i = 0; i < (int)(blockDim.x >> 5); ++i) r = fmax(r, sh[i]);
   return r;
 }
-// sum partials[k*nb .. k*nb+nb) -> out[k], for k < nk (one block per k)
-__global__ void k_finish_sum(const double *part, int nb, double *out, int nk) {
-  __shared__ double sh[32];
-  const int k = blockIdx.x;
-  double v = 0;
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) v += part[(long)k * nb + i];
-  double r = block_sum(v, sh);
-  if (threadIdx.x == 0 && k < nk) out[k] = r;
-}
-
 // Reductions finished by the kernel that produces them: each block reduces
 // its threads' v[k] (a sum, or a max for the bits of MAXMASK), writes its
 // partials part[k*gridDim + block], and the last block to arrive (an atomic
@@ -1129,63 +1119,6 @@ __global__ void k_nl_energy_d(int nproj, int nstate, const int *proj_isa, const 
 }
 
 // ---------------------------------------------------------------- forces
-// e_sr (total_energy.f90:133-239) with minimum image (nlp = 0); one block.
-// F(3,na_max,nsp) zeroed first as in the reference; esr -> out[0].
-__global__ void k_esr(int nsp, const int *na, int na_max, const int *zv, const double *atco, double alat, int sym,
-                      int tfor, double *F, double *out) {
-  const double pi = 4.0 * atan(1.0);
-  const double rckj = sqrt(1.2 * 1.2 + 1.2 * 1.2);
-  double esr = 0;
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 3 * na_max * nsp; ++k) F[k] = 0.0;
-  __syncthreads();
-  // serial over pairs in thread 0 for the force accumulation order; the
-  // pair count is O(atoms^2) and small
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < nsp; ++k)
-      for (int j = k; j < nsp; ++j) {
-        double zv2 = (double)(zv[k] * zv[j]);
-        if (fabs(zv2) < 1e-10) continue;
-        for (int l = 0; l < na[k]; ++l)
-          for (int m = (k == j) ? l + 1 : 0; m < na[j]; ++m) {
-            const double *xl = atco + 3 * (l + (long)na_max * k), *xm = atco + 3 * (m + (long)na_max * j);
-            double x1 = xl[0] - xm[0], y1 = xl[1] - xm[1], z1 = xl[2] - xm[2], X, Y, Z;
-            if (sym == 1) {
-              double A = alat, h = A / 2.0;
-              X = fmod(x1, A); Y = fmod(y1, A); Z = fmod(z1, A);
-              X = X - A * trunc(X / h); Y = Y - A * trunc(Y / h); Z = Z - A * trunc(Z / h);
-            } else {
-              double ma = alat * sqrt(2.0) / 4.0, s2 = sqrt(2.0);
-              X = (x1 + y1) / s2; Y = (-x1 + y1) / s2;
-              X = fmod(X, 2.0 * ma); Y = fmod(Y, 2.0 * ma);
-              Z = fmod(z1, 2.0 * ma * s2);
-              X = X - 2.0 * ma * trunc(X / ma); Y = Y - 2.0 * ma * trunc(Y / ma);
-              Z = Z - 2.0 * ma * s2 * trunc(Z / (s2 * ma));
-              if (!(fabs(X) + fabs(Y) + s2 * fabs(Z) < 2.0 * ma)) {
-                X = X - copysign(ma, X); Y = Y - copysign(ma, Y); Z = Z - copysign(s2 * ma, Z);
-              }
-              double xt = (X - Y) / s2;
-              Y = (X + Y) / s2;
-              X = xt;
-            }
-            double e2 = X * X + Y * Y + Z * Z, r = sqrt(e2), arg = r / rckj;
-            if (arg <= 20.0) {
-              double add = zv2 * erfc(arg) / r;
-              esr += add;
-              if (tfor) {
-                double pre = (2.0 * zv2 / sqrt(pi)) * exp(-arg * arg) / rckj;
-                double rep = (add + pre) / e2;
-                double *fl = F + 3 * (l + (long)na_max * k), *fm = F + 3 * (m + (long)na_max * j);
-                fl[0] += rep * X; fl[1] += rep * Y; fl[2] += rep * Z;
-                fm[0] -= rep * X; fm[1] -= rep * Y; fm[2] -= rep * Z;
-              }
-            }
-          }
-      }
-    out[0] = esr;
-  }
-}
-
 // POTFOR (nuclear_grad.f90:4-50): per atom and block partial sums of
 // Re[S_I(G) (rhos V_H(G)* + vps rho_e(G)*) i G] 2 Omega tpiba over G != 0
 __global__ void k_potfor(int ngrho, const int *inyh, int nh1, int nh2, int nh3, AtomArgs aa, const double *hg,
