@@ -2551,7 +2551,7 @@ int amdk_scf_iteration(amdk_ctx *c, int istep, double gcut, amdk_energies *e, do
   cudaSetDevice(c->device);
   const int q = (c->precision == AMDK_MIXED) ? 1 : 0;
   // graphs from the second iteration on, once this precision has run eagerly
-  // (first-call setup of kernels and cuBLAS stays out of the capture)
+  // (the kernels' first-call setup stays out of the capture)
   const bool graph = c->use_graphs && istep > 1 && c->warm[q];
   c->h_pin[S_NSCAL] = (double)istep;  // copied by segment A (copy_istep)
   cudaEventRecord(c->ev0, c->st);

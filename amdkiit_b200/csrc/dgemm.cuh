@@ -1,5 +1,5 @@
 // FP64 products of the band space on the FP64 tensor cores (DMMA,
-// mma.sync.m8n8k4.f64), fed by TMA: the FP64 path's overlap S = 2 C0^T C0
+// mma.sync.m16n8k8.f64), fed by TMA: the FP64 path's overlap S = 2 C0^T C0
 // (ortho_gs DSYRK, wfn_initialize.f90:481), Lambda = 2 C2^T C0 (OVLAP_D,
 // wfn_initialize.f90:234-263), the projections nl = 2 P^T C0
 // (pseudopotential.f90:211-213) and dfnl = 2 tpiba Q^T C0

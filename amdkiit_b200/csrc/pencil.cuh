@@ -348,6 +348,20 @@ constexpr int pencil_blocks(size_t csize, int nt) { return csize == 16 ? 512 / n
 constexpr int pencil_tiles(int nc, int w) { return w > 0 ? (nc + w - 1) / w : 4096; }
 // V(r)psi.  The whole plane (GA = 1) where a tile then still keeps half of a
 // block's threads busy, else one group of its columns at a time.
+// Both sides of the rules, 64 pairs, us a launch, the rule's choice first:
+//   whole plane | groups   FP64 100^3 473 | 580, 128^3 1001 | 1225; FP32 100^3
+//     241 | 296, 160^3 1099 | 1222; at every length the whole plane is faster,
+//     by 2% (48^3 FP64) to 77% (108^3 FP32).  FP64 160^3: groups 3155 | 4548.
+//   256 threads | 512   FP64 36^3 30 | 41, 60^3 115 | 134, 72^3 185 | 223,
+//     96^3 431 | 430; FP32 36^3 19 | 24, 60^3 70 | 76, 72^3 100 | 109, 96^3
+//     235 | 217
+//   512 threads | 256   FP64 48^3 71 | 60, 64^3 123 | 107, 80^3 269 | 252, 90^3
+//     395 | 391, 100^3 473 | 494, 108^3 639 | 685; FP32 48^3 40 | 36, 64^3
+//     66 | 60, 80^3 137 | 139, 90^3 205 | 209, 100^3 241 | 255, 108^3 340 | 357,
+//     120^3 434 | 479, 128^3 497 | 687.  The count of busy threads misses what
+//     else the smaller blocks bring at 48, 64 and 80 and cost at 96.
+//   FP32 of 512 threads: two blocks at 144^3 745 | one 797, one at 160^3 1099 |
+//     two 1775
 template <typename C, int N> struct VpsiShape {
   static constexpr int N1 = fft_n1(N), N2 = N / N1;
   static constexpr size_t cs = sizeof(C);
@@ -367,6 +381,27 @@ template <typename C, int N> struct VpsiShape {
 // Z2 values per thread: long second phases take the split of the z transform
 // the other way round (Z1 x Z2), and where the sums take more than 20
 // registers a block of 512 FP32 threads has the SM to itself.
+// Both sides of the rules, 64 pairs, us a launch with its reduction, the rule's
+// choice first:
+//   256 threads | 512   FP64 36^3 32 | 44, 48^3 46 | 65, 64^3 73 | 93; FP32 36^3
+//     26 | 30, 48^3 34 | 41, 64^3 49 | 58
+//   512 threads | 256   FP64 60^3 96 | 91, 72^3 141 | 144, 80^3 180 | 178, 90^3
+//     322 | 307, 96^3 341 | 286, 100^3 305 | 307, 108^3 537 | 486, 120^3
+//     630 | 564, 128^3 660 | 675, 144^3 945 | 1114, 160^3 1734 | 5494; FP32 60^3
+//     61 | 61, 72^3 85 | 83, 80^3 105 | 101, 90^3 188 | 184, 96^3 247 | 166,
+//     100^3 181 | 185, 108^3 285 | 300, 120^3 409 | 337, 128^3 338 | 363, 144^3
+//     575 | 612, 160^3 997 | 804
+//   two FP32 blocks of 512 | one   60^3 61 | 71, 72^3 85 | 96, 80^3 105 | 120,
+//     90^3 188 | 208, 100^3 181 | 197, 108^3 285 | 392, 128^3 338 | 433
+//   one FP32 block of 512 | two   96^3 247 | 202, 120^3 409 | 355, 144^3
+//     575 | 521, 160^3 997 | 854: above 20 sums two blocks spill and are faster
+//     all the same, so the bound of 20 holds back these four lengths
+//   z split swapped | as it is   128^3 FP64 660 | 665, FP32 338 | 430; 160^3
+//     1734 | 1915, 997 | 1012
+//   z split as it is | swapped   FP64 72^3 141 | 146, 90^3 322 | 337, 96^3
+//     341 | 371, 120^3 630 | 636; FP32 72^3 85 | 85, 90^3 188 | 193, 108^3
+//     285 | 288, 96^3 247 | 187, 120^3 409 | 346 (at these two the swap also
+//     takes the sums from 24 to under 20)
 template <typename C, int N> struct DensShape {
   static constexpr size_t cs = sizeof(C);
   static constexpr int GA = col_groups(N), GC = N / GA;

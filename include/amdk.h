@@ -216,8 +216,8 @@ int amdk_fft_sphere(amdk_ctx *ctx, int sign, double *coef, double *grid);
 int amdk_profile(amdk_ctx *ctx, int enable);
 int amdk_profile_get(amdk_ctx *ctx, int kind, long *launches, double *total_ms, double *bytes);
 
-/* Number of this library's kernels launched so far on the context (cuBLAS
- * kernels are not counted). */
+/* Number of this library's kernels launched so far on the context (copies and
+ * memsets are not counted). */
 int amdk_launch_count(amdk_ctx *ctx, long *n);
 
 /* amdk_fft_sphere for callers that cannot allocate device memory (an
