@@ -2101,6 +2101,7 @@ struct amdk_slab {
   double *d_hg = nullptr, *d_rhopart = nullptr;
   void *d_vp = nullptr, *d_pscr = nullptr;
   int pos_T = -1;
+  cudaEvent_t ev_caller = nullptr;  // the legacy default stream's work before a call on the context's stream
   std::vector<void *> allocs;
   template <typename T> int alloc(T **p, size_t n) {
     RC(dalloc(p, n));
@@ -2113,6 +2114,7 @@ struct amdk_slab {
     return 0;
   }
   ~amdk_slab() {
+    if (ev_caller) cudaEventDestroy(ev_caller);
     for (void *p : allocs) cudaFree(p);
   }
 };
@@ -2132,6 +2134,7 @@ static int slab_create(amdk_ctx *c, int nranks, int rank, amdk_slab *s) {
     set_error("slab decomposition: rank out of range");
     return AMDK_ERR_BADARG;
   }
+  CK(cudaEventCreateWithFlags(&s->ev_caller, cudaEventDisableTiming));
   const int n1 = h.nr[0], n2 = h.nr[1];
   std::vector<int> ray_ky, ray_kz, posp, posm, owner;
   ray_tables(h, ray_ky, ray_kz, posp, posm);
@@ -2207,8 +2210,16 @@ static int slab_create(amdk_ctx *c, int nranks, int rank, amdk_slab *s) {
   return 0;
 }
 
-static cudaStream_t slab_stream(const amdk_slab *s, void *stream) {
-  return stream ? (cudaStream_t)stream : s->c->st;
+// The call's stream, or (NULL) the context's.  That one is non-blocking, so it
+// is put behind what the caller has queued on the legacy default stream (a
+// program whose arrays live there, torch's default for one, passes NULL).
+static int slab_stream(const amdk_slab *s, void *stream, cudaStream_t *st) {
+  *st = stream ? (cudaStream_t)stream : s->c->st;
+  if (!stream) {
+    CK(cudaEventRecord(s->ev_caller, cudaStreamLegacy));
+    CK(cudaStreamWaitEvent(*st, s->ev_caller, 0));
+  }
+  return 0;
 }
 static int slab_check_pairs(const amdk_slab *s, int band0, int npairs) {
   const int nst = s->c->nstate;
@@ -3025,7 +3036,8 @@ int amdk_slab_pairs_out(amdk_slab *s, const double *c0, int band0, int npairs, v
   if (!s || !c0 || !send) return AMDK_ERR_BADARG;
   RC(slab_check_pairs(s, band0, npairs));
   CK(cudaSetDevice(s->c->device));
-  const cudaStream_t st = slab_stream(s, stream);
+  cudaStream_t st;
+  RC(slab_stream(s, stream, &st));
   if (s->precision == AMDK_MIXED) RC(slab_pairs_out_t<float2>(s, (const double2 *)c0, band0, npairs, (float2 *)send, st));
   else RC(slab_pairs_out_t<double2>(s, (const double2 *)c0, band0, npairs, (double2 *)send, st));
   return slab_finish(s, stream);
@@ -3035,7 +3047,8 @@ int amdk_slab_planes_vpsi(amdk_slab *s, void *recv, int npairs, const double *v,
   if (!s || !recv || !v) return AMDK_ERR_BADARG;
   RC(slab_check_pairs(s, 0, npairs));
   CK(cudaSetDevice(s->c->device));
-  const cudaStream_t st = slab_stream(s, stream);
+  cudaStream_t st;
+  RC(slab_stream(s, stream, &st));
   if (s->precision == AMDK_MIXED) RC(slab_vpsi_t<float2>(s, (float2 *)recv, npairs, v, st));
   else RC(slab_vpsi_t<double2>(s, (double2 *)recv, npairs, v, st));
   return slab_finish(s, stream);
@@ -3046,7 +3059,8 @@ int amdk_slab_planes_density(amdk_slab *s, const void *recv, int band0, int npai
   if (!s || !recv || !rho) return AMDK_ERR_BADARG;
   RC(slab_check_pairs(s, band0, npairs));
   CK(cudaSetDevice(s->c->device));
-  const cudaStream_t st = slab_stream(s, stream);
+  cudaStream_t st;
+  RC(slab_stream(s, stream, &st));
   if (s->precision == AMDK_MIXED) RC(slab_density_t<float2>(s, (const float2 *)recv, band0, npairs, rho, accumulate, st));
   else RC(slab_density_t<double2>(s, (const double2 *)recv, band0, npairs, rho, accumulate, st));
   return slab_finish(s, stream);
@@ -3056,7 +3070,8 @@ int amdk_slab_pairs_in(amdk_slab *s, void *back, const double *c0, int band0, in
   if (!s || !back || !c0 || !c2) return AMDK_ERR_BADARG;
   RC(slab_check_pairs(s, band0, npairs));
   CK(cudaSetDevice(s->c->device));
-  const cudaStream_t st = slab_stream(s, stream);
+  cudaStream_t st;
+  RC(slab_stream(s, stream, &st));
   if (s->precision == AMDK_MIXED)
     RC(slab_pairs_in_t<float2>(s, (float2 *)back, (const double2 *)c0, band0, npairs, (double2 *)c2, st));
   else RC(slab_pairs_in_t<double2>(s, (double2 *)back, (const double2 *)c0, band0, npairs, (double2 *)c2, st));
@@ -3070,7 +3085,8 @@ int amdk_slab_gram(amdk_slab *s, const double *a, const double *b, int n, double
   }
   amdk_ctx *c = s->c;
   CK(cudaSetDevice(c->device));
-  const cudaStream_t st = slab_stream(s, stream);
+  cudaStream_t st;
+  RC(slab_stream(s, stream, &st));
   if (s->ng == 0) {
     CK(cudaMemsetAsync(out, 0, sizeof(double) * n * n, st));
     CK(cudaStreamSynchronize(st));

@@ -296,7 +296,8 @@ int amdk_ensemble_destroy(amdk_ensemble *ens);
  *                            FFT(V psi)) on the rank's G vectors (vpsi,
  *                            wfn_initialize.f90:283-362, without fnonloc)
  * Pointers are device pointers; stream: a cudaStream_t to launch on
- * (asynchronous), or NULL for the context's stream with the call waited for.
+ * (asynchronous), or NULL for the context's stream, after the work queued on
+ * the legacy default stream and with the call waited for.
  * A slab object serves one call at a time.  Closed-shell systems on grids
  * with the pencil transforms only; nranks <= 16. */
 #define AMDK_SLAB_MAXRANKS 16

@@ -7,6 +7,7 @@ import pytest
 from amdkiit_b200 import configs
 from amdkiit_b200.engine import FP64, MIXED, Engine, Ensemble
 from amdkiit_b200.inputs import XC_PBE
+from amdkiit_b200.slab import LocalExchange, Slab, apply_local_h, density, gram
 from tests.helpers import start_coefficients
 
 pytestmark = pytest.mark.gpu
@@ -79,5 +80,57 @@ def test_ensemble_after_work_on_the_members_streams(prec):
         ens.close()
         for e in members:
             e.close()
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("prec", [FP64, MIXED])
+def test_slab_calls_follow_the_default_stream(prec):
+    """The slab entries called without a stream run on the context's own, which
+    does not wait for the default stream by itself: inputs written there, and
+    the exchange's copies there, are complete before a kernel reads them, also
+    when the default stream is 10 ms behind."""
+    import torch
+
+    class Exchange(LocalExchange):
+        def __init__(self, late):
+            self.late = late
+
+        def __call__(self, sends, send_counts, recv_counts):
+            if self.late:
+                torch.cuda._sleep(20_000_000)
+            return super().__call__(sends, send_counts, recv_counts)
+
+    s = configs.small_water()
+    e = _engine(s, prec)
+    slabs = [Slab(e, 2, r) for r in range(2)]
+    c0 = e.get_wfn()
+    start = [torch.from_numpy(np.ascontiguousarray(c0[:, x.local_g])).cuda() for x in slabs]
+    vs = [torch.randn(x.grid, dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(x.rank))
+          for x in slabs]
+    torch.cuda.synchronize()
+    got = []
+    for late in (False, True):
+        c0s = [torch.zeros_like(c) for c in start]
+        c2s, rhos = [torch.zeros_like(c) for c in start], [torch.zeros_like(v) for v in vs]
+        torch.cuda.synchronize()
+        ex = Exchange(late)
+        if late:
+            torch.cuda._sleep(20_000_000)
+        for c, x in zip(c0s, start):
+            c.copy_(x)
+        if not late:
+            torch.cuda.synchronize()
+        out = [gram(slabs, ex, c0s, c0s, e.nstate)[0]]
+        if late:
+            for c in c0s:
+                torch.cuda._sleep(20_000_000)
+                c.mul_(1.0)
+        apply_local_h(slabs, ex, c0s, vs, c2s)
+        density(slabs, ex, c0s, rhos)
+        torch.cuda.synchronize()
+        got.append([x.cpu().numpy() for x in out + c2s + rhos])
+    for x in slabs:
+        x.close()
     for a, b in zip(*got):
         assert np.array_equal(a, b)
