@@ -170,6 +170,7 @@ struct amdk_ctx {
   CUtensorMap tm_p_tn, tm_q_tn;
   CUtensorMap tm_a_tn, tm_b_tn, tm_a_nn, tm_s_nn;
   bool warm[2] = {false, false};  // an eager iteration has run at this pair precision
+  bool queued = true;             // an entry may have left work on the context stream
   void *c0_first = nullptr;       // the buffer that held C0 at creation
   // BOMD predictor: converged C0 of earlier steps, most recent first
   static constexpr int MAX_PRED = 8;
@@ -2335,6 +2336,13 @@ static int slab_pairs_in_t(amdk_slab *s, C *back, const double2 *c0, int band0, 
   return 0;
 }
 
+// Start of an entry that puts work on the context stream, which it may leave
+// there; amdk_scf_iteration waits for the stream and clears the mark.
+static void enter(amdk_ctx *c) {
+  cudaSetDevice(c->device);
+  c->queued = true;
+}
+
 extern "C" {
 
 const char *amdk_last_error(void) { return g_err.c_str(); }
@@ -2475,13 +2483,13 @@ int amdk_set_precision(amdk_ctx *c, int precision) {
 
 int amdk_set_positions(amdk_ctx *c, const double *atco) {
   if (!c || !atco) return AMDK_ERR_BADARG;
-  cudaSetDevice(c->device);
+  enter(c);
   return do_positions(c, atco);
 }
 
 int amdk_set_wfn(amdk_ctx *c, const double *c0) {
   if (!c || !c0) return AMDK_ERR_BADARG;
-  cudaSetDevice(c->device);
+  enter(c);
   // on the context stream (after any kernel still reading or writing C0, e.g.
   // the rotation of an ortho that returned), and complete before returning
   CK(cudaMemcpyAsync(c->d_c0, c0, sizeof(double2) * (size_t)c->hs.ngpw * c->nstate, cudaMemcpyHostToDevice, c->st));
@@ -2496,7 +2504,7 @@ int amdk_set_density(amdk_ctx *c, const double *rho) {
     set_error("amdk_set_density: the open-shell branch keeps a density per spin; not supported");
     return AMDK_ERR_UNSUPPORTED;
   }
-  cudaSetDevice(c->device);
+  enter(c);
   const size_t npt = (size_t)c->hs.nr[0] * c->hs.nr[1] * c->hs.nr[2];
   CK(cudaMemcpyAsync(c->d_rho, rho, sizeof(double) * npt, cudaMemcpyHostToDevice, c->st));
   if (c->precision == AMDK_MIXED) RC(rhor2g_t<float2>(c));
@@ -2507,7 +2515,7 @@ int amdk_set_density(amdk_ctx *c, const double *rho) {
 
 int amdk_get_wfn(amdk_ctx *c, double *c0) {
   if (!c || !c0) return AMDK_ERR_BADARG;
-  cudaSetDevice(c->device);
+  enter(c);
   CK(cudaStreamSynchronize(c->st));
   CK(cudaMemcpy(c0, c->d_c0, sizeof(double2) * (size_t)c->hs.ngpw * c->nstate, cudaMemcpyDeviceToHost));
   return 0;
@@ -2515,32 +2523,32 @@ int amdk_get_wfn(amdk_ctx *c, double *c0) {
 
 int amdk_ortho(amdk_ctx *c) {
   if (!c) return AMDK_ERR_BADARG;
-  cudaSetDevice(c->device);
+  enter(c);
   return do_ortho(c);
 }
 int amdk_density(amdk_ctx *c) {
   if (!c) return AMDK_ERR_BADARG;
-  cudaSetDevice(c->device);
+  enter(c);
   return do_density(c);
 }
 int amdk_potential(amdk_ctx *c) {
   if (!c) return AMDK_ERR_BADARG;
-  cudaSetDevice(c->device);
+  enter(c);
   return do_potential(c);
 }
 int amdk_energy(amdk_ctx *c, amdk_energies *e) {
   if (!c) return AMDK_ERR_BADARG;
-  cudaSetDevice(c->device);
+  enter(c);
   return do_energy(c, e);
 }
 int amdk_apply_h(amdk_ctx *c) {
   if (!c) return AMDK_ERR_BADARG;
-  cudaSetDevice(c->device);
+  enter(c);
   return do_apply_h(c);
 }
 int amdk_gradient(amdk_ctx *c, double *gemax) {
   if (!c) return AMDK_ERR_BADARG;
-  cudaSetDevice(c->device);
+  enter(c);
   RC(do_gradient(c));
   if (gemax) {
     CK(cudaMemcpyAsync(gemax, c->d_scal + S_GMAX, sizeof(double), cudaMemcpyDeviceToHost, c->st));
@@ -2550,7 +2558,7 @@ int amdk_gradient(amdk_ctx *c, double *gemax) {
 }
 int amdk_pcg(amdk_ctx *c, int istep) {
   if (!c || istep < 1) return AMDK_ERR_BADARG;
-  cudaSetDevice(c->device);
+  enter(c);
   ++c->nlaunch;
   k_set_scalar<<<1, 1, 0, c->st>>>(c->d_scal + S_ISTEP, (double)istep);  // by value: this entry returns without a wait
   gmax_precon(c);  // the caller may have changed C2 since the gradient
@@ -2559,7 +2567,7 @@ int amdk_pcg(amdk_ctx *c, int istep) {
 
 int amdk_scf_iteration(amdk_ctx *c, int istep, double gcut, amdk_energies *e, double *gemax, int *converged) {
   if (!c || istep < 1) return AMDK_ERR_BADARG;
-  cudaSetDevice(c->device);
+  enter(c);
   const int q = (c->precision == AMDK_MIXED) ? 1 : 0;
   // graphs from the second iteration on, once this precision has run eagerly
   // (the kernels' first-call setup stays out of the capture)
@@ -2579,6 +2587,7 @@ int amdk_scf_iteration(amdk_ctx *c, int istep, double gcut, amdk_energies *e, do
   else RC(seg_b());
   cudaEventRecord(c->ev1, c->st);
   CK(cudaEventSynchronize(c->ev1));
+  c->queued = false;
   float ms = 0;
   cudaEventElapsedTime(&ms, c->ev0, c->ev1);
   c->last_ms = ms;
@@ -2672,10 +2681,10 @@ int amdk_ensemble_iteration(amdk_ensemble *E, const int *istep, double gcut, amd
   // work that a member's earlier entries left on its stream (an ortho's
   // rotation, a CG update) comes first
   for (amdk_ctx *c : E->m)
-    if (cudaStreamQuery(c->st) != cudaSuccess) {
-      cudaGetLastError();  // not ready
+    if (c->queued) {
       CK(cudaEventRecord(c->ev0, c->st));
       CK(cudaStreamWaitEvent(E->st, c->ev0, 0));
+      c->queued = false;
     }
   CK(cudaEventRecord(E->ev0, E->st));
   RC(run_all(false));
@@ -2703,7 +2712,7 @@ int amdk_ensemble_last_ms(amdk_ensemble *E, double *ms) {
 
 int amdk_ionic_forces(amdk_ctx *c, double *force) {
   if (!c || !force) return AMDK_ERR_BADARG;
-  cudaSetDevice(c->device);
+  enter(c);
   // forces of the current C0: density (for POTFOR) and projections with
   // H nl (NLFOR)
   RC(do_density(c));
@@ -2728,7 +2737,7 @@ int amdk_wfn_set_predictor(amdk_ctx *c, int npoints, const double *coef) {
 
 int amdk_wfn_extrapolate(amdk_ctx *c) {
   if (!c) return AMDK_ERR_BADARG;
-  cudaSetDevice(c->device);
+  enter(c);
   const HostSetup &h = c->hs;
   const size_t cw = (size_t)h.ngpw * c->nstate;
   const int keep = c->pred_npts - 1;  // earlier steps the predictor uses
@@ -2776,7 +2785,7 @@ int amdk_wfn_history_clear(amdk_ctx *c) {
 
 int amdk_backward(amdk_ctx *c, double *dE_dR, double *dE_dpsi) {
   if (!c || (!dE_dR && !dE_dpsi)) return AMDK_ERR_BADARG;
-  cudaSetDevice(c->device);
+  enter(c);
   const HostSetup &h = c->hs;
   RC(do_density(c));
   if (dE_dpsi) RC(do_potential(c));
@@ -2801,7 +2810,7 @@ int amdk_backward(amdk_ctx *c, double *dE_dR, double *dE_dpsi) {
 
 int amdk_get_array(amdk_ctx *c, const char *name, void *dst, size_t bytes) {
   if (!c || !name || !dst) return AMDK_ERR_BADARG;
-  cudaSetDevice(c->device);
+  enter(c);
   const HostSetup &h = c->hs;
   long npt = (long)h.nr[0] * h.nr[1] * h.nr[2];
   const void *src = nullptr;
@@ -2838,7 +2847,7 @@ int amdk_get_array(amdk_ctx *c, const char *name, void *dst, size_t bytes) {
 
 int amdk_fft_sphere(amdk_ctx *c, int sign, double *coef, double *grid) {
   if (!c || !coef || !grid || (sign != 1 && sign != -1)) return AMDK_ERR_BADARG;
-  cudaSetDevice(c->device);
+  enter(c);
   const HostSetup &h = c->hs;
   long npt = (long)h.nr[0] * h.nr[1] * h.nr[2];
   if (sign == -1) {
@@ -2860,7 +2869,7 @@ int amdk_fft_sphere(amdk_ctx *c, int sign, double *coef, double *grid) {
 
 int amdk_profile(amdk_ctx *c, int enable) {
   if (!c) return AMDK_ERR_BADARG;
-  cudaSetDevice(c->device);
+  enter(c);
   CK(cudaStreamSynchronize(c->st));
   prof_harvest(c);
   c->prof = enable != 0;
@@ -2874,7 +2883,7 @@ int amdk_profile(amdk_ctx *c, int enable) {
 
 int amdk_profile_get(amdk_ctx *c, int kind, long *launches, double *total_ms, double *bytes) {
   if (!c || kind < 0 || kind >= KT_N) return AMDK_ERR_BADARG;
-  cudaSetDevice(c->device);
+  enter(c);
   CK(cudaStreamSynchronize(c->st));
   prof_harvest(c);
   if (launches) *launches = c->kt_count[kind];
