@@ -72,3 +72,27 @@ def test_sphere_transform_matches_numpy(n):
     back, _ = e.fft_sphere(+1, grid=ref)
     assert np.abs(back - coef).max() < 1e-11 * np.abs(coef).max()
     e.close()
+
+
+@pytest.mark.parametrize("prec", [FP64, MIXED])
+@pytest.mark.parametrize("box,ecut,nr", [((9.0, 11.0, 12.0), 42.0, (40, 48, 50)), ((12.0, 8.5, 15.0), 40.0, (50, 36, 64))])
+def test_three_different_lengths(box, ecut, nr, prec):
+    """An orthorhombic cell: every axis with a length of its own, known at
+    compile time or not, through the slab passes."""
+    s = configs.cluster(1, 9.0, 77, ecut=ecut)
+    s = dataclasses.replace(s, a_cell=np.diag(box), alat=box[0], xc=XC_PBE)
+    o, e = Oracle(s, 0), Engine(s, prec)
+    assert e.nr == nr
+    o.set_wfn(start_coefficients(o.gvectors()["hg"][: o.ngpw], o.d("tpiba"), o.nstate))
+    assert o.ortho() == 0
+    for r in ("eval_density", "rhor2g", "eval_pot", "cal_vpot_ex", "pp_energy", "vpsi", "fnonloc"):
+        o.call(r)
+    e.set_wfn(o.c0())
+    e.density()
+    e.potential()
+    e.energy()
+    e.apply_h()
+    errs = {"rho": _rel(e.get("rho"), o.real_grid("rho")), "v_pot": _rel(e.get("v_pot"), o.real_grid("v_pot")),
+            "c2": _rel(e.get("c2"), o.c2())}
+    e.close()
+    assert max(errs.values()) < BAR[prec], errs
