@@ -126,3 +126,26 @@ def test_orthonormalisation_does_not_depend_on_the_scale(power):
         out.append(e.get_wfn())
     e.close()
     assert _rel(out[1], out[0]) < 1e-11
+
+
+def test_reciprocal_square_root_of_a_pivot():
+    """One band: U^-1 is the pivot's reciprocal square root (the hardware's
+    approximation and two Newton steps), so C0 U^-1 over C0 shows it.  Over the
+    binades from 2^-1000 to 2^200 it is within 1 ulp, the bound of CUDA's own
+    rsqrt: 2^-52, and 2^-53 for the product's rounding."""
+    s = _hydrogens(1)
+    e = Engine(s, FP64)
+    c = _start(e, s)
+    rng = np.random.default_rng(5)
+    worst = 0.0
+    for power in np.concatenate([rng.uniform(-500.0, 100.0, 200), rng.uniform(-451.0, -449.0, 40)]):
+        x = c * 2.0 ** power
+        e.set_wfn(x)
+        e.ortho()
+        exact = np.longdouble(1.0) / np.sqrt(np.longdouble(e.get("overlap")[0, 0]))
+        y = e.get_wfn()
+        big = np.abs(x.real) > 0.1 * np.abs(x.real).max()
+        ratio = np.longdouble(y.real[big]) / (np.longdouble(x.real[big]) * exact)
+        worst = max(worst, float(np.abs(ratio - 1).max()))
+    e.close()
+    assert worst <= 2.0 ** -52 + 2.0 ** -53, worst
