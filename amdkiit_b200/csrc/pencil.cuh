@@ -377,41 +377,48 @@ template <typename C, int N> struct VpsiShape {
   static constexpr int MINB = small ? pencil_blocks(cs, 256) : (wl == w2 ? pencil_blocks(cs, 512) : 1);
   static constexpr size_t smem = pencil_smem_bytes(cs, N, GC | 1, W);
 };
-// Density: one column group at a time.  Its sums stay in registers, NS tiles x
-// Z2 values per thread: long second phases take the split of the z transform
-// the other way round (Z1 x Z2), and where the sums take more than 20
-// registers a block of 512 FP32 threads has the SM to itself.
+// Density: one column group at a time, or the whole plane where three groups
+// would read and transform its rays three times and the whole plane's sums are
+// no more than 20.  The sums stay in registers, NS tiles x Z2 values per thread:
+// long second phases take the split of the z transform the other way round
+// (Z1 x Z2), where the sums take more than 20 registers a block of 512 FP32
+// threads has the SM to itself, and blocks of 256 take more than 20 only where
+// a larger block would leave over two fifths of its threads idle (96 points).
 // Both sides of the rules, 64 pairs, us a launch with its reduction, the rule's
 // choice first:
-//   256 threads | 512   FP64 36^3 32 | 44, 48^3 46 | 65, 64^3 73 | 93; FP32 36^3
-//     26 | 30, 48^3 34 | 41, 64^3 49 | 58
-//   512 threads | 256   FP64 60^3 96 | 91, 72^3 141 | 144, 80^3 180 | 178, 90^3
-//     322 | 307, 96^3 341 | 286, 100^3 305 | 307, 108^3 537 | 486, 120^3
-//     630 | 564, 128^3 660 | 675, 144^3 945 | 1114, 160^3 1734 | 5494; FP32 60^3
-//     61 | 61, 72^3 85 | 83, 80^3 105 | 101, 90^3 188 | 184, 96^3 247 | 166,
-//     100^3 181 | 185, 108^3 285 | 300, 120^3 409 | 337, 128^3 338 | 363, 144^3
-//     575 | 612, 160^3 997 | 804
+//   256 threads | 512   FP64 36^3 32 | 44, 48^3 46 | 65, 64^3 73 | 93, 96^3
+//     286 | 341; FP32 36^3 26 | 30, 48^3 34 | 41, 64^3 49 | 58, 96^3 166 | 247
+//   512 threads | 256   FP64 60^3 96 | 91, 72^3 141 | 144, 80^3 180 | 178, 100^3
+//     305 | 307, 108^3 537 | 486, 120^3 630 | 564, 128^3 660 | 675, 144^3
+//     945 | 1114, 160^3 1734 | 5494; FP32 60^3 61 | 61, 72^3 85 | 83, 80^3
+//     105 | 101, 100^3 181 | 185, 108^3 285 | 300, 120^3 409 | 337, 128^3
+//     338 | 363, 144^3 575 | 612, 160^3 997 | 804 (with 4 pairs 256 threads take
+//     2 to 8% more at 120 and 160)
+//   the whole density call: whole plane | three groups   90^3 FP64 64 pairs
+//     316 | 408, 16 pairs 120 | 137, 4 pairs 68 | 69; FP32 198 | 255, 87 | 97,
+//     61 | 60.  Three groups | whole plane   108^3 FP64 736 | 625, 229 | 211,
+//     110 | 107; FP32 387 | 341, 141 | 145, 77 | 97
 //   two FP32 blocks of 512 | one   60^3 61 | 71, 72^3 85 | 96, 80^3 105 | 120,
-//     90^3 188 | 208, 100^3 181 | 197, 108^3 285 | 392, 128^3 338 | 433
-//   one FP32 block of 512 | two   96^3 247 | 202, 120^3 409 | 355, 144^3
-//     575 | 521, 160^3 997 | 854: above 20 sums two blocks spill and are faster
-//     all the same, so the bound of 20 holds back these four lengths
+//     100^3 181 | 197, 108^3 285 | 392, 128^3 338 | 433
+//   one FP32 block of 512 | two   120^3 409 | 355, 144^3 575 | 521, 160^3
+//     997 | 854: above 20 sums two blocks spill and are faster all the same where
+//     there are many pairs
 //   z split swapped | as it is   128^3 FP64 660 | 665, FP32 338 | 430; 160^3
 //     1734 | 1915, 997 | 1012
-//   z split as it is | swapped   FP64 72^3 141 | 146, 90^3 322 | 337, 96^3
-//     341 | 371, 120^3 630 | 636; FP32 72^3 85 | 85, 90^3 188 | 193, 108^3
-//     285 | 288, 96^3 247 | 187, 120^3 409 | 346 (at these two the swap also
-//     takes the sums from 24 to under 20)
+//   z split as it is | swapped   FP64 72^3 141 | 146, 120^3 630 | 636; FP32 72^3
+//     85 | 85, 108^3 285 | 288, 120^3 409 | 346 (there the swap also takes the
+//     sums from 24 to 20)
 template <typename C, int N> struct DensShape {
   static constexpr size_t cs = sizeof(C);
-  static constexpr int GA = col_groups(N), GC = N / GA;
   static constexpr bool swap = N / fft_n1(N) > 12;
   static constexpr int Z1 = swap ? N / fft_n1(N) : fft_n1(N), Z2 = N / Z1, ZM = Z1 > Z2 ? Z1 : Z2;
+  static constexpr int whole = pencil_width(cs, N, N, 512, pencil_blocks(cs, 512), ZM);
+  static constexpr int GA = col_groups(N) == 3 && pencil_tiles(N, whole) * Z2 <= 20 ? 1 : col_groups(N), GC = N / GA;
   static constexpr int w2 = pencil_width(cs, N, GC, 512, pencil_blocks(cs, 512), ZM),
                        ws = pencil_width(cs, N, GC, 256, pencil_blocks(cs, 256), ZM);
   static constexpr bool two = w2 > 0 && (cs == 16 || pencil_tiles(GC, w2) * Z2 <= 20);
   static constexpr int wl = two ? w2 : pencil_width(cs, N, GC, 512, 1, ZM);
-  static constexpr bool small = ws > 0 && pencil_tiles(GC, ws) * Z2 <= 20 &&
+  static constexpr bool small = ws > 0 && (pencil_tiles(GC, ws) * Z2 <= 20 || 5 * wl * ZM < 3 * 512) &&
                                 20 * pencil_tiles(GC, wl) * 512 >= 21 * pencil_tiles(GC, ws) * 256;
   static constexpr int NT = small ? 256 : 512, W = small ? ws : wl, NS = pencil_tiles(GC, W);
   static constexpr int MINB = small ? pencil_blocks(cs, 256) : (two ? pencil_blocks(cs, 512) : 1);

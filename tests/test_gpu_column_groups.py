@@ -64,7 +64,7 @@ def test_two_spins(n, prec):
 
 
 @pytest.mark.parametrize("prec", [FP64, MIXED])
-@pytest.mark.parametrize("n,nranks", [(72, 3), (160, 1), (160, 3)])
+@pytest.mark.parametrize("n,nranks", [(72, 3), (90, 3), (96, 2), (160, 1), (160, 3)])
 def test_ray_segments(n, nranks, prec):
     import torch
     box = 13.0 if n < 100 else 24.0
